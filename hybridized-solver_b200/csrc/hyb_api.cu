@@ -2,6 +2,7 @@
 // the level schedule (captured into CUDA graphs), plain FP64 and mixed FP32+refinement
 // solves.
 #include "hyb_internal.h"
+#include "hyb_front.cuh"
 #include "hyb_kernels.cuh"
 #include "hyb_krylov.cuh"
 #include "hyb_pivot.cuh"
@@ -532,6 +533,36 @@ template <typename T> bool inverse_pivots(const hyb_system *h, int64_t l)
     return std::is_same_v<T, float> && fused_pivots(sh) && sh.piv64 && mode64 == 2 && tc_level<T>(h, l) && h->d_dinv;
 }
 
+// Whether a level's pivots take k_front: all of up to 128 rows, except where an option asks for
+// one of the 64-row kernels by name (HYB_OPTION_ROW_PIVOTS, HYB_OPTION_PIVOT_LU_ONCE).
+bool front_pivots(const hyb_system *h, const Symbolic::LevelShape &sh)
+{
+    if (sh.max_piv > hyb::kFrontMax)
+        return false;
+    return !fused_pivots(sh) || (h->lu_once < 0 && h->row_pivots < 0);
+}
+
+// LU and row solves of level l's pivots by k_front.
+template <typename T> int enqueue_front(hyb_system *h, T *slab, int64_t l, cudaStream_t st, uint64_t &launches)
+{
+    const Symbolic &S = h->S;
+    const int64_t p0 = S.lvl_ptr[l], p1 = S.lvl_ptr[l + 1];
+    const Symbolic::LevelShape &sh = S.shape[l];
+    const float glim = std::is_same_v<T, float> ? h->growth_limit : 0.0f;
+    const int64_t units = S.lu_pref[p1] - S.lu_pref[p0];
+    // A strip of 64 columns takes as long again as the factorization beside it, so where SMs are
+    // idle the strips are narrower: 16 or 32 columns while every CTA still has an SM.
+    int strip = 64;
+    while (strip > 16 && units * ((sh.max_up + strip / 2 - 1) / (strip / 2)) <= sm_count())
+        strip /= 2;
+    const dim3 grid((unsigned)units, (unsigned)std::max(1, (sh.max_up + strip - 1) / strip));
+    hyb::k_front<T><<<grid, hyb::kFrontThreads, hyb::front_smem(sh.max_piv), st>>>(h->ds, slab, p0, p1, h->d_lu_tickets,
+                                                                                 h->d_status, glim, strip);
+    ++launches;
+    HYB_LAUNCHED("k_front", l);
+    return enqueue_split<T>(h, slab, l, st, launches);
+}
+
 // With pair_first (level l's pivot is the first of a pair on the inverse-and-products path),
 // the first pivot's update of the second one's row and column is applied by the products
 // kernel too; the caller then issues no separate update for it.
@@ -631,7 +662,7 @@ int enqueue_pivots(hyb_system *h, T *slab, int64_t l, cudaStream_t st, uint64_t 
         HYB_LAUNCHED("k_piv64", l);
         return HYB_SUCCESS;
     }
-    if (fused_pivots(sh))
+    if (fused_pivots(sh) && !front_pivots(h, sh))
     {
         // fused: diagonal LU (padded to 64x64) and the solves of the pivot rows' upper blocks;
         // pivots of up to 32 rows stay on the generic kernels, whose serial steps are short
@@ -678,6 +709,8 @@ int enqueue_pivots(hyb_system *h, T *slab, int64_t l, cudaStream_t st, uint64_t 
         HYB_LAUNCHED("k_lu_trsm64", l);
         return enqueue_split<T>(h, slab, l, st, launches);
     }
+    if (front_pivots(h, sh))
+        return enqueue_front<T>(h, slab, l, st, launches);
     const int lu_bytes = lu_smem_bytes<T>(sh.max_piv);
     int *hg = glim > 0 ? h->d_hg : nullptr;
     if (lu_bytes <= optin)
@@ -2385,6 +2418,8 @@ HYB_API int hyb_decompose(hyb_system *h, int precision, hyb_decompose_info *info
             allow_smem(hyb::k_piv64_inv, hyb::kInvSmem),
             allow_smem(hyb::k_strips64_inv, hyb::kInvSmem),
             allow_smem(hyb::k_split64, 0),
+            allow_smem(hyb::k_front<double>, hyb::front_smem(hyb::kFrontMax)),
+            allow_smem(hyb::k_front<float>, hyb::front_smem(hyb::kFrontMax)),
             allow_smem(hyb::k_update<double>, 0),
             allow_smem(hyb::k_update<float>, 0),
             allow_smem(hyb::k_update32<double>, 0),

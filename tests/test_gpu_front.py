@@ -1,0 +1,101 @@
+"""k_front: LU of a pivot block and the solves of its row's upper blocks, FP64 inside."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from conftest import rel_err
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _dense_blocks(sizes, seed, scale=1.0):
+    """Every block of a block-dense, diagonally dominant system."""
+    from hybsol.b200.meshgen import _assemble
+
+    rng = np.random.default_rng(seed)
+    sizes = np.asarray(sizes, dtype=np.int64)
+    keys = [(i, j) for i in range(len(sizes)) for j in range(len(sizes))]
+    vals = []
+    for i, j in keys:
+        v = rng.standard_normal((sizes[i], sizes[j])) / np.sqrt(sizes[j])
+        vals.append(scale * (v + (2 * len(sizes) * np.eye(sizes[i]) if i == j else 0)))
+    return _assemble(sizes, np.array([k[0] for k in keys]), np.array([k[1] for k in keys]), vals)
+
+
+def _factors(ns, mat):
+    return [[ns.get_block(i, c, (int(mat.sizes[i]), int(mat.sizes[c]))) for c in ns.row_cols(i)] for i in range(mat.n_blocks)]
+
+
+# edges of the 8-column panels, of the 16-row padding, of a warp's rows, of the 16/32/64-column
+# strips (70 and 130 wide upper blocks) and of the largest pivot the kernel takes (128)
+@pytest.mark.parametrize("m", [1, 7, 8, 9, 16, 17, 32, 33, 63, 64, 65, 96, 127, 128, 129])
+def test_pivot_sizes_match_oracle(gpu, m):
+    mat = _dense_blocks([m, 70, m, 130, 3], seed=m)
+    osys = O.OracleSystem.from_csr(mat.sizes, mat.row_ptr, mat.cols, mat.vals)
+    osys.decompose()
+    ns = gpu.NativeSystem.from_matrix(mat)
+    info = ns.decompose(gpu.FP64)
+    assert info["zero_pivots"] == 0 and info["non_finite"] == 0
+    f64 = _factors(ns, mat)
+    for i, row in enumerate(f64):
+        for c, got in enumerate(row):
+            assert rel_err(got, osys.get_block(i, c)) < 1e-12, (i, c)
+    # FP32 factors: every stored value is rounded once per pivot that updates it, five times at most
+    ns.set_option(gpu.OPTION_BLOCK_SCALING, 0)
+    info = ns.decompose(gpu.MIXED)
+    assert info["growth_fp64"] == 0 and info["growth_kept"] == 0
+    for row, ref in zip(_factors(ns, mat), f64):
+        for got, want in zip(row, ref):
+            assert rel_err(got, want) < 1e-4
+
+
+def test_many_pivots_of_a_level_match_oracle(gpu):
+    """Pivots of different sizes, with and without upper blocks, in one launch."""
+    from hybsol.b200 import meshgen
+
+    mat = meshgen.block_diagonal([_dense_blocks(s, seed=k) for k, s in enumerate([[5], [40, 3], [64, 64], [9, 100, 2], [128], [17, 65]])])
+    osys = O.OracleSystem.from_csr(mat.sizes, mat.row_ptr, mat.cols, mat.vals)
+    osys.decompose()
+    ns = gpu.NativeSystem.from_matrix(mat)
+    ns.decompose(gpu.FP64)
+    for i in range(mat.n_blocks):
+        for c in ns.row_cols(i):
+            got = ns.get_block(i, c, (int(mat.sizes[i]), int(mat.sizes[c])))
+            assert rel_err(got, osys.get_block(i, c)) < 1e-12, (i, c)
+
+
+@pytest.mark.parametrize("exponent", [-1004, 1015])
+def test_extreme_pivots(gpu, exponent):
+    """A power of two scales the lower and the upper parts exactly and leaves the quotients
+    alone, also where a pivot's reciprocal overflows or loses digits (its values, at least
+    2^-1018 here, stay 2^56 above the smallest spacing: 1e-13 leaves room for the roundings)."""
+    sizes = [20, 9, 70]
+    ref, mat = _dense_blocks(sizes, seed=4), _dense_blocks(sizes, seed=4, scale=2.0**exponent)
+    ns, na = gpu.NativeSystem.from_matrix(mat), gpu.NativeSystem.from_matrix(ref)
+    ns.decompose(gpu.FP64)
+    na.decompose(gpu.FP64)
+    for i in range(len(sizes)):
+        for c in range(len(sizes)):
+            got, want = (s.get_block(i, c, (sizes[i], sizes[c])) for s in (ns, na))
+            if i < c:
+                assert rel_err(got, want) < 1e-13
+            elif i > c:
+                assert rel_err(got * 2.0**-exponent, want) < 1e-13
+            else:
+                assert rel_err(np.tril(got, -1), np.tril(want, -1)) < 1e-13
+                assert rel_err(np.triu(got) * 2.0**-exponent, np.triu(want)) < 1e-13
+
+
+def test_overflowing_quotient_stays_infinite(gpu):
+    """1e200 / 1e-200 is infinite by division; the reciprocal's product corrected by its residual
+    would be NaN."""
+    from hybsol.b200.meshgen import _assemble
+
+    d = np.array([[1e-200, 0.0], [1e200, 1.0]])
+    mat = _assemble(np.array([2]), np.array([0]), np.array([0]), [d])
+    ns = gpu.NativeSystem.from_matrix(mat)
+    ns.decompose(gpu.FP64)
+    assert ns.get_block(0, 0, (2, 2))[1, 0] == np.inf
