@@ -6,6 +6,7 @@
 #include "hyb_kernels.cuh"
 #include "hyb_krylov.cuh"
 #include "hyb_pivot.cuh"
+#include "hyb_solve.cuh"
 #include "hyb_umma.cuh"
 
 #include "hybsol_b200.h"
@@ -212,16 +213,16 @@ struct hyb_system
     double *d_a = nullptr; // original values (FP64, CSR order)
     int *d_status = nullptr;
     int *d_tickets = nullptr; // per pivot: partial products of the solve stage already published
-    // dataflow solve: per block row the tag of the last solve direction that finished it,
-    // the solve's status words, and the partial products of every pivot (flow_nrhs columns)
-    int *d_flags = nullptr;
-    int *d_pflags = nullptr; // per pivot: tag of the solve direction whose early partials are summed
     int *d_lu_tickets = nullptr; // per pivot: CTAs of k_lu_trsm64 that have read the diagonal block
     int *d_solve_status = nullptr;
+    // dataflow solve: the tagged vectors and partial sums of k_flow (flow_nrhs columns), and the tags' epoch
     uint32_t solve_epoch = 0;
-    double *d_flow64 = nullptr;
-    float *d_flow32 = nullptr;
+    hyb::Tagged<double> *d_flow64 = nullptr;
+    hyb::Tagged<float> *d_flow32 = nullptr;
     int64_t flow64_nrhs = 0, flow32_nrhs = 0;
+    // D^{-1} L of the late blocks (Symbolic::w_off), in the factors' precision
+    double *d_w64 = nullptr;
+    float *d_w32 = nullptr;
     int factored = -1; // -1, HYB_PRECISION_FP64 or HYB_PRECISION_MIXED
     double *d_f64 = nullptr;
     float *d_f32 = nullptr;
@@ -281,8 +282,8 @@ struct hyb_system
         cudaFree(d_a);
         cudaFree(d_status);
         cudaFree(d_tickets);
-        cudaFree(d_flags);
-        cudaFree(d_pflags);
+        cudaFree(d_w64);
+        cudaFree(d_w32);
         cudaFree(d_lu_tickets);
         cudaFree(d_solve_status);
         cudaFree(d_flow64);
@@ -405,13 +406,16 @@ int upload_symbolic(hyb_system *h)
         {S.upd2_pref.data(), S.upd2_pref.size() * 8, (const void **)&d.upd2_pref},
         {S.split_pref.data(), S.split_pref.size() * 8, (const void **)&d.split_pref},
         {S.tc_pref.data(), S.tc_pref.size() * 8, (const void **)&d.tc_pref},
-        {S.fwd_pref.data(), S.fwd_pref.size() * 8, (const void **)&d.fwd_pref},
         {S.fwdu_pref.data(), S.fwdu_pref.size() * 8, (const void **)&d.fwdu_pref},
         {S.fwd_item_p.data(), S.fwd_item_p.size() * 4, (const void **)&d.fwd_item_p},
         {S.bwd_item_p.data(), S.bwd_item_p.size() * 4, (const void **)&d.bwd_item_p},
         {S.bwd_first.data(), S.bwd_first.size() * 8, (const void **)&d.bwd_first},
         {S.fwd_rows.data(), S.fwd_rows.size() * 8, (const void **)&d.fwd_rows},
         {S.bwd_rows.data(), S.bwd_rows.size() * 8, (const void **)&d.bwd_rows},
+        {S.w_off.data(), S.w_off.size() * 8, (const void **)&d.w_off},
+        {S.w_row.data(), S.w_row.size() * 4, (const void **)&d.w_row},
+        {S.w_blk.data(), S.w_blk.size() * 4, (const void **)&d.w_blk},
+        {S.w_out.data(), S.w_out.size() * 8, (const void **)&d.w_out},
         {S.inv_idx.data(), S.inv_idx.size() * 4, (const void **)&d.inv_idx},
         {S.inv_row.data(), S.inv_row.size() * 4, (const void **)&d.inv_row},
         {S.mt_tgt.data(), S.mt_tgt.size() * 4, (const void **)&d.mt_tgt},
@@ -771,6 +775,32 @@ template <typename T> int enqueue_inverses(hyb_system *h, T *slab, uint64_t &lau
         ++launches;
         HYB_LAUNCHED("k_diag_inv64", h->S.n_levels - 1);
     }
+    return HYB_SUCCESS;
+}
+
+template <typename T> T *&late_blocks(hyb_system *h);
+template <> double *&late_blocks<double>(hyb_system *h)
+{
+    return h->d_w64;
+}
+template <> float *&late_blocks<float>(hyb_system *h)
+{
+    return h->d_w32;
+}
+
+// W of the solves' late blocks, in one launch once the factors are final.
+template <typename T> int enqueue_late(hyb_system *h, T *slab, uint64_t &launches)
+{
+    const Symbolic &S = h->S;
+    if (S.w_blk.empty())
+        return HYB_SUCCESS;
+    int m = 0;
+    for (int32_t k : S.w_row)
+        m = std::max(m, S.size[k]);
+    const dim3 grid((unsigned)S.w_blk.size(), (unsigned)((S.w_cols + 63) / 64));
+    hyb::k_late<T><<<grid, hyb::kFrontThreads, hyb::front_smem(m), h->stream>>>(h->ds, slab, late_blocks<T>(h));
+    ++launches;
+    HYB_LAUNCHED("k_late", S.n_levels - 1);
     return HYB_SUCCESS;
 }
 
@@ -1147,7 +1177,8 @@ template <typename T> int enqueue_factor(hyb_system *h, T *slab, uint64_t &launc
         HYB_CUDA(cudaEventRecord(h->ev_join, st2));
         HYB_CUDA(cudaStreamWaitEvent(st, h->ev_join, 0));
     }
-    if ((rc = enqueue_inverses<T>(h, slab, launches)) != HYB_SUCCESS)
+    if ((rc = enqueue_inverses<T>(h, slab, launches)) != HYB_SUCCESS ||
+        (rc = enqueue_late<T>(h, slab, launches)) != HYB_SUCCESS)
         return rc;
     HYB_CUDA(cudaGetLastError());
     return HYB_SUCCESS;
@@ -1162,42 +1193,6 @@ template <typename T> const T *solve_dinv(const hyb_system *h)
         return nullptr;
 }
 
-// Forward + backward substitution of y (type V, dof x nrhs) with the factors in `slab`.
-template <typename T, typename V> int enqueue_solve(hyb_system *h, const T *slab, V *y, V *scratch, int nrhs,
-                                                    uint64_t &launches)
-{
-    const Symbolic &S = h->S;
-    const T *dinv = solve_dinv<T>(h);
-    const DevSym &ds = h->ds;
-    cudaStream_t st = h->stream;
-    // tickets return to zero after every stage; clearing them guards against an aborted solve
-    HYB_CUDA(cudaMemsetAsync(h->d_tickets, 0, S.n * sizeof(int), st));
-    for (int64_t l = 0; l < S.n_levels; ++l)
-    {
-        const int64_t p0 = S.lvl_ptr[l], p1 = S.lvl_ptr[l + 1];
-        const int64_t units = S.fwdu_pref[p1] - S.fwdu_pref[p0];
-        const int mp = S.shape[l].max_piv;
-        const int acc_bytes = (mp * nrhs * (int)sizeof(V) + 15) / 16 * 16;
-        const int diag_bytes = mp * (mp | 1) * (int)sizeof(T);
-        const int stage = acc_bytes + diag_bytes <= solve_smem_cap() ? 1 : 0;
-        hyb::k_fwd_stage<T, V><<<(unsigned)units, hyb::kThreads, acc_bytes + (stage ? diag_bytes : 0), st>>>(
-            ds, slab, y, scratch, h->d_tickets, p0, p1, nrhs, stage, dinv);
-        ++launches;
-    }
-    for (int64_t l = S.n_levels - 1; l >= 0; --l)
-    {
-        const int64_t p0 = S.lvl_ptr[l], p1 = S.lvl_ptr[l + 1];
-        const int64_t units = S.trsm_pref[p1] - S.trsm_pref[p0];
-        if (units == 0)
-            continue;
-        hyb::k_bwd_stage<T, V><<<(unsigned)units, hyb::kThreads, 0, st>>>(ds, slab, y, scratch, h->d_tickets, p0,
-                                                                         p1, nrhs);
-        ++launches;
-    }
-    HYB_CUDA(cudaGetLastError());
-    return HYB_SUCCESS;
-}
-
 // Largest diagonal block of the system.
 int max_pivot(const Symbolic &S)
 {
@@ -1207,80 +1202,134 @@ int max_pivot(const Symbolic &S)
     return m;
 }
 
-template <typename V> V *&flow_scratch(hyb_system *h);
-template <> double *&flow_scratch<double>(hyb_system *h)
+// Shared memory of the substitution kernels for nc right-hand sides at a time; `stage` is set where the
+// largest diagonal block fits beside their vectors.
+template <typename T> int64_t solve_smem(const Symbolic &S, int nc, int &stage)
+{
+    const int mp = max_pivot(S);
+    stage = hyb::flow_smem_bytes<T>(mp, nc, true) <= solve_smem_cap() ? 1 : 0;
+    return hyb::flow_smem_bytes<T>(mp, nc, stage != 0);
+}
+
+// Right-hand sides that a CTA of the substitution kernels takes at a time.
+constexpr int kSolveColumns = 4;
+
+template <typename T, int NC>
+int enqueue_stages(hyb_system *h, const T *slab, T *y, T *scratch, int nrhs, uint64_t &launches)
+{
+    const Symbolic &S = h->S;
+    const T *dinv = solve_dinv<T>(h), *wbuf = late_blocks<T>(h);
+    cudaStream_t st = h->stream;
+    int stage = 0;
+    const int64_t smem = solve_smem<T>(S, NC, stage);
+    const int mp = max_pivot(S);
+    if (smem > solve_smem_cap())
+        return HYB_TOO_LARGE;
+    HYB_CUDA(allow_smem(hyb::k_stage<T, NC, true>, (int)smem));
+    HYB_CUDA(allow_smem(hyb::k_stage<T, NC, false>, (int)smem));
+    for (int64_t l = 0; l < S.n_levels; ++l)
+    {
+        const int64_t p0 = S.lvl_ptr[l], first = S.fwdu_pref[p0], units = S.fwdu_pref[S.lvl_ptr[l + 1]] - first;
+        hyb::k_stage<T, NC, true><<<(unsigned)units, hyb::kThreads, (size_t)smem, st>>>(
+            h->ds, slab, wbuf, y, scratch, h->d_tickets, dinv, first, S.fwd_rows[p0], nrhs, mp, stage);
+        ++launches;
+    }
+    for (int64_t l = S.n_levels - 1; l >= 0; --l)
+    {
+        const int64_t p0 = S.lvl_ptr[l], first = S.bwd_lvl[l];
+        const int64_t units = (l > 0 ? S.bwd_lvl[l - 1] : (int64_t)S.bwd_item_p.size()) - first;
+        if (S.trsm_pref[S.lvl_ptr[l + 1]] == S.trsm_pref[p0])
+            continue; // no upper blocks
+        hyb::k_stage<T, NC, false><<<(unsigned)units, hyb::kThreads, (size_t)smem, st>>>(
+            h->ds, slab, wbuf, y, scratch, h->d_tickets, dinv, first, S.bwd_rows[p0], nrhs, mp, stage);
+        ++launches;
+    }
+    HYB_CUDA(cudaGetLastError());
+    return HYB_SUCCESS;
+}
+
+// Forward + backward substitution of y (dof x nrhs) with the factors in `slab`, one launch per
+// level and direction.
+template <typename T>
+int enqueue_solve(hyb_system *h, const T *slab, T *y, T *scratch, int nrhs, uint64_t &launches)
+{
+    // tickets return to zero after every stage; clearing them guards against an aborted solve
+    HYB_CUDA(cudaMemsetAsync(h->d_tickets, 0, h->S.n * sizeof(int), h->stream));
+    return nrhs == 1 ? enqueue_stages<T, 1>(h, slab, y, scratch, nrhs, launches)
+                     : enqueue_stages<T, kSolveColumns>(h, slab, y, scratch, nrhs, launches);
+}
+
+template <typename T> hyb::Tagged<T> *&flow_scratch(hyb_system *h);
+template <> hyb::Tagged<double> *&flow_scratch<double>(hyb_system *h)
 {
     return h->d_flow64;
 }
-template <> float *&flow_scratch<float>(hyb_system *h)
+template <> hyb::Tagged<float> *&flow_scratch<float>(hyb_system *h)
 {
     return h->d_flow32;
+}
+
+template <typename T, int NC, bool kFwd>
+int launch_flow(hyb_system *h, const T *slab, T *y, hyb::Tagged<T> *scr, int tag, int nrhs)
+{
+    const Symbolic &S = h->S;
+    int stage = 0, per_sm = 0;
+    const int64_t smem = solve_smem<T>(S, NC, stage);
+    if (smem > solve_smem_cap())
+        return HYB_TOO_LARGE;
+    HYB_CUDA(allow_smem(hyb::k_flow<T, NC, kFwd>, (int)smem));
+    HYB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hyb::k_flow<T, NC, kFwd>, hyb::kThreads,
+                                                           (size_t)smem));
+    if (per_sm < 1)
+        return HYB_TOO_LARGE;
+    const int64_t len = S.dof_off[S.n] * nrhs;
+    DevSym ds = h->ds;
+    const T *wbuf = late_blocks<T>(h), *dinv = solve_dinv<T>(h);
+    hyb::Tagged<T> *ytag = scr, *ztag = scr + len, *ptag = scr + 2 * len;
+    int64_t items = (int64_t)(kFwd ? S.fwd_item_p.size() : S.bwd_item_p.size()), withhold = kFwd ? h->withhold_slot : -1;
+    int mp = max_pivot(S), *status = h->d_solve_status;
+    uint64_t wait_ns = h->wait_ns;
+    void *args[] = {&ds,  (void *)&slab, &wbuf, &y,  &ytag,  &ztag,     &ptag,   &dinv,
+                    &tag, &items,        &nrhs, &mp, &stage, &withhold, &status, &wait_ns};
+    const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(items, (int64_t)per_sm * sm_count()));
+    HYB_CUDA(cudaLaunchCooperativeKernel((const void *)hyb::k_flow<T, NC, kFwd>, dim3(grid), dim3(hyb::kThreads), args,
+                                         (size_t)smem, h->stream));
+    return HYB_SUCCESS;
 }
 
 // Dataflow substitution of y (dof x nrhs) with the factors in `slab`: one cooperative
 // launch per direction. Returns HYB_TOO_LARGE (before anything is enqueued) when the
 // device cannot keep a useful grid resident, in which case the caller uses the staged solve.
-template <typename T, typename V> int enqueue_solve_flow(hyb_system *h, const T *slab, V *y, int nrhs, uint64_t &launches)
+template <typename T> int enqueue_solve_flow(hyb_system *h, const T *slab, T *y, int nrhs, uint64_t &launches)
 {
     const Symbolic &S = h->S;
-    const int mp = max_pivot(S);
-    const int acc_bytes = (mp * nrhs * (int)sizeof(V) + 15) / 16 * 16;
-    const int diag_bytes = mp * (mp | 1) * (int)sizeof(T);
-    int stage = acc_bytes + diag_bytes <= solve_smem_cap() ? 1 : 0;
-    const int fwd_smem = acc_bytes + (stage ? diag_bytes : 0);
-    int per_sm_f = 0, per_sm_b = 0, coop = 0, dev = 0;
+    int coop = 0, dev = 0;
     HYB_CUDA(cudaGetDevice(&dev));
     HYB_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-    HYB_CUDA(cudaFuncSetAttribute(hyb::k_fwd_flow<T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, fwd_smem));
-    HYB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_f, hyb::k_fwd_flow<T, V>, hyb::kThreads, fwd_smem));
-    HYB_CUDA(cudaFuncSetAttribute(hyb::k_bwd_flow<T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, acc_bytes));
-    HYB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_b, hyb::k_bwd_flow<T, V>, hyb::kThreads, acc_bytes));
-    if (!coop || per_sm_f < 1 || per_sm_b < 1)
+    if (!coop)
         return HYB_TOO_LARGE;
-    V *&scr = flow_scratch<V>(h);
-    int64_t &have = std::is_same_v<V, double> ? h->flow64_nrhs : h->flow32_nrhs;
+    hyb::Tagged<T> *&scr = flow_scratch<T>(h);
+    int64_t &have = std::is_same_v<T, double> ? h->flow64_nrhs : h->flow32_nrhs;
     if (have < nrhs)
     {
         cudaFree(scr);
         scr = nullptr;
         have = 0;
-        const int64_t rows = std::max<int64_t>(1, std::max(S.fwd_rows[S.n], S.bwd_rows[S.n]));
-        HYB_CUDA(cudaMalloc(&scr, rows * nrhs * sizeof(V)));
+        const int64_t words = (2 * S.dof_off[S.n] + std::max(S.fwd_rows[S.n], S.bwd_rows[S.n])) * nrhs;
+        HYB_CUDA(cudaMalloc(&scr, words * sizeof(hyb::Tagged<T>)));
+        HYB_CUDA(cudaMemsetAsync(scr, 0, words * sizeof(hyb::Tagged<T>), h->stream)); // no solve has the tag 0
         have = nrhs;
     }
-    cudaStream_t st = h->stream;
-    HYB_CUDA(cudaMemsetAsync(h->d_tickets, 0, S.n * sizeof(int), st));
-    if (h->withhold_slot >= 0)
-    {
-        // the pivot's early-partial ticket starts far past its count, so no CTA ever takes
-        // the last one: the pre-sum is never released and the finisher's wait runs out
-        static const int kPoison = 1 << 30;
-        HYB_CUDA(cudaMemcpyAsync(h->d_tickets + h->withhold_slot, &kPoison, sizeof(int), cudaMemcpyHostToDevice, st));
-    }
-    h->solve_epoch = (h->solve_epoch + 1) & 0x3fffffffu;
-    int tag_f = (int)(2 * h->solve_epoch + 1), tag_b = tag_f + 1;
-    DevSym ds = h->ds;
-    V *scratch = scr;
-    int *tickets = h->d_tickets, *flags = h->d_flags, *pflags = h->d_pflags, *status = h->d_solve_status;
-    const T *dinv = solve_dinv<T>(h);
-    uint64_t wait_ns = h->wait_ns;
-    int64_t nf = (int64_t)S.fwd_item_p.size(), nb = (int64_t)S.bwd_item_p.size();
-    const int sms = sm_count();
-    {
-        const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(nf, (int64_t)per_sm_f * sms));
-        void *args[] = {&ds,    (void *)&slab, &y,    &scratch, &tickets, &flags,  &pflags,
-                        &tag_f, &nf,           &nrhs, &stage,   &dinv,    &status, &wait_ns};
-        HYB_CUDA(cudaLaunchCooperativeKernel((const void *)hyb::k_fwd_flow<T, V>, dim3(grid), dim3(hyb::kThreads),
-                                             args, fwd_smem, st));
-    }
-    {
-        const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(nb, (int64_t)per_sm_b * sms));
-        void *args[] = {&ds, (void *)&slab, &y, &scratch, &tickets, &flags, &pflags, &tag_b, &nb, &nrhs, &status, &wait_ns};
-        HYB_CUDA(cudaLaunchCooperativeKernel((const void *)hyb::k_bwd_flow<T, V>, dim3(grid), dim3(hyb::kThreads),
-                                             args, acc_bytes, st));
-    }
+    h->solve_epoch = (h->solve_epoch + 1) & 0x1fffffffu;
+    const int tag = (int)(2 * h->solve_epoch + 1);
+    int rc = nrhs == 1 ? launch_flow<T, 1, true>(h, slab, y, scr, tag, nrhs)
+                       : launch_flow<T, kSolveColumns, true>(h, slab, y, scr, tag, nrhs);
+    if (rc != HYB_SUCCESS)
+        return rc;
+    rc = nrhs == 1 ? launch_flow<T, 1, false>(h, slab, y, scr, tag + 1, nrhs)
+                   : launch_flow<T, kSolveColumns, false>(h, slab, y, scr, tag + 1, nrhs);
     launches += 2;
-    return HYB_SUCCESS;
+    return rc;
 }
 
 // Runs `body` (which enqueues work and counts launches) through a cached CUDA graph.
@@ -1316,18 +1365,18 @@ template <typename F> int run_graph(hyb_system *h, std::unique_ptr<GraphExec> &s
 
 // One substitution of y with the factors in `slab`: the dataflow form when it is enabled
 // and the device can run it, else the staged form through the cached graph `slot`.
-template <typename T, typename V>
-int substitute(hyb_system *h, const T *slab, V *y, V *scratch, int nrhs, std::unique_ptr<GraphExec> &slot)
+template <typename T>
+int substitute(hyb_system *h, const T *slab, T *y, T *scratch, int nrhs, std::unique_ptr<GraphExec> &slot)
 {
     if (h->flow)
     {
         uint64_t count = 0;
-        const int rc = enqueue_solve_flow<T, V>(h, slab, y, nrhs, count);
+        const int rc = enqueue_solve_flow<T>(h, slab, y, nrhs, count);
         h->last_launches += count;
         if (rc != HYB_TOO_LARGE)
             return rc;
     }
-    return run_graph(h, slot, [&](uint64_t &count) { return enqueue_solve<T, V>(h, slab, y, scratch, nrhs, count); });
+    return run_graph(h, slot, [&](uint64_t &count) { return enqueue_solve<T>(h, slab, y, scratch, nrhs, count); });
 }
 
 int ensure_solve_buffers(hyb_system *h, int64_t nrhs)
@@ -1506,7 +1555,7 @@ int apply_factors(hyb_system *h, const double *v, double *z, int nr, uint64_t &c
         else
             hyb::k_convert<double, float><<<eg, hyb::kThreads, 0, h->stream>>>(v, h->d_yf, len);
         auto &slot = h->g_solve[{HYB_PRECISION_MIXED, nr}];
-        const int rc = substitute<float, float>(h, h->d_f32, h->d_yf, h->d_scr32, nr, slot);
+        const int rc = substitute<float>(h, h->d_f32, h->d_yf, h->d_scr32, nr, slot);
         if (rc != HYB_SUCCESS)
             return rc;
         if (h->factors_scaled)
@@ -1519,7 +1568,7 @@ int apply_factors(hyb_system *h, const double *v, double *z, int nr, uint64_t &c
     if (z != v)
         HYB_CUDA(cudaMemcpyAsync(z, v, len * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
     auto &slot = h->g_solve[{HYB_PRECISION_FP64, nr}];
-    return substitute<double, double>(h, h->d_f64, z, h->d_scr64, nr, slot);
+    return substitute<double>(h, h->d_f64, z, h->d_scr64, nr, slot);
 }
 
 struct RefineResult
@@ -1887,7 +1936,7 @@ int solve_host_once(hyb_system *h, const double *in, double *out, bool transpose
         rc = run_graph(h, h->g_solveT[1],
                        [&](uint64_t &c) { return enqueue_solve_transpose(h, h->d_x, h->d_tscr, 1, c); });
     else
-        rc = substitute<double, double>(h, h->d_f64, h->d_x, h->d_scr64, 1, h->g_solve[{HYB_PRECISION_FP64, 1}]);
+        rc = substitute<double>(h, h->d_f64, h->d_x, h->d_scr64, 1, h->g_solve[{HYB_PRECISION_FP64, 1}]);
     if (rc != HYB_SUCCESS)
         return rc;
     int sst[hyb::ST_WORDS];
@@ -2072,10 +2121,6 @@ HYB_API int hyb_system_create(uint64_t n, const uint64_t *block_sizes, const uin
     HYB_CUDA(cudaMemsetAsync(h->d_a, 0, std::max<int64_t>(1, h->S.a_val_off.back()) * sizeof(double), h->stream));
     HYB_CUDA(cudaMalloc(&h->d_status, hyb::ST_WORDS * sizeof(int)));
     HYB_CUDA(cudaMalloc(&h->d_tickets, h->S.n * sizeof(int)));
-    HYB_CUDA(cudaMalloc(&h->d_flags, h->S.n * sizeof(int)));
-    HYB_CUDA(cudaMemsetAsync(h->d_flags, 0, h->S.n * sizeof(int), h->stream));
-    HYB_CUDA(cudaMalloc(&h->d_pflags, h->S.n * sizeof(int)));
-    HYB_CUDA(cudaMemsetAsync(h->d_pflags, 0, h->S.n * sizeof(int), h->stream));
     HYB_CUDA(cudaMalloc(&h->d_lu_tickets, h->S.n * sizeof(int)));
     HYB_CUDA(cudaMemsetAsync(h->d_lu_tickets, 0, h->S.n * sizeof(int), h->stream));
     HYB_CUDA(cudaMalloc(&h->d_solve_status, hyb::ST_WORDS * sizeof(int)));
@@ -2135,10 +2180,6 @@ HYB_API int hyb_system_copy(const hyb_system *src, hyb_system **out)
     HYB_CUDA(cudaMalloc(&h->d_a, a_bytes));
     HYB_CUDA(cudaMalloc(&h->d_status, hyb::ST_WORDS * sizeof(int)));
     HYB_CUDA(cudaMalloc(&h->d_tickets, h->S.n * sizeof(int)));
-    HYB_CUDA(cudaMalloc(&h->d_flags, h->S.n * sizeof(int)));
-    HYB_CUDA(cudaMemsetAsync(h->d_flags, 0, h->S.n * sizeof(int), h->stream));
-    HYB_CUDA(cudaMalloc(&h->d_pflags, h->S.n * sizeof(int)));
-    HYB_CUDA(cudaMemsetAsync(h->d_pflags, 0, h->S.n * sizeof(int), h->stream));
     HYB_CUDA(cudaMalloc(&h->d_lu_tickets, h->S.n * sizeof(int)));
     HYB_CUDA(cudaMemsetAsync(h->d_lu_tickets, 0, h->S.n * sizeof(int), h->stream));
     HYB_CUDA(cudaMalloc(&h->d_solve_status, hyb::ST_WORDS * sizeof(int)));
@@ -2155,6 +2196,16 @@ HYB_API int hyb_system_copy(const hyb_system *src, hyb_system **out)
     {
         HYB_CUDA(cudaMalloc(&h->d_f32, slab * sizeof(float)));
         HYB_CUDA(cudaMemcpyAsync(h->d_f32, src->d_f32, slab * sizeof(float), cudaMemcpyDeviceToDevice, h->stream));
+    }
+    if (src->d_w64)
+    {
+        HYB_CUDA(cudaMalloc(&h->d_w64, std::max<int64_t>(1, h->S.w_elems) * sizeof(double)));
+        HYB_CUDA(cudaMemcpyAsync(h->d_w64, src->d_w64, h->S.w_elems * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
+    }
+    if (src->d_w32)
+    {
+        HYB_CUDA(cudaMalloc(&h->d_w32, std::max<int64_t>(1, h->S.w_elems) * sizeof(float)));
+        HYB_CUDA(cudaMemcpyAsync(h->d_w32, src->d_w32, h->S.w_elems * sizeof(float), cudaMemcpyDeviceToDevice, h->stream));
     }
     if (src->d_dinv)
     {
@@ -2401,8 +2452,8 @@ HYB_API int hyb_decompose(hyb_system *h, int precision, hyb_decompose_info *info
             allow_smem(hyb::k_lu<float, true>, optin),
             allow_smem(hyb::k_trsm<double, true>, optin),
             allow_smem(hyb::k_trsm<float, true>, optin),
-            allow_smem(hyb::k_fwd_stage<double, double>, optin),
-            allow_smem(hyb::k_fwd_stage<float, float>, optin),
+            allow_smem(hyb::k_late<double>, hyb::front_smem(hyb::kFlowLateMax)),
+            allow_smem(hyb::k_late<float>, hyb::front_smem(hyb::kFlowLateMax)),
             allow_smem(hyb::k_update64_f64<0>, hyb::kUpd64Smem),
             allow_smem(hyb::k_update64_f64<1>, hyb::kUpd64Smem),
             allow_smem(hyb::k_update64_f64<2>, hyb::kUpd64Smem),
@@ -2450,14 +2501,17 @@ HYB_API int hyb_decompose(hyb_system *h, int precision, hyb_decompose_info *info
         {
             cudaFree(h->d_f32);
             cudaFree(h->d_dinv);
+            cudaFree(h->d_w32);
             h->d_f32 = nullptr;
             h->d_dinv = nullptr;
+            h->d_w32 = nullptr;
             h->g_factor[1].reset();
             h->g_solve.clear();
         }
         if (!h->d_f64)
         {
             HYB_CUDA(cudaMalloc(&h->d_f64, slab * sizeof(double)));
+            HYB_CUDA(cudaMalloc(&h->d_w64, std::max<int64_t>(1, S.w_elems) * sizeof(double)));
             h->g_factor[0].reset();
             h->g_solve.clear();
         }
@@ -2485,13 +2539,16 @@ HYB_API int hyb_decompose(hyb_system *h, int precision, hyb_decompose_info *info
         if (h->d_f64)
         {
             cudaFree(h->d_f64);
+            cudaFree(h->d_w64);
             h->d_f64 = nullptr;
+            h->d_w64 = nullptr;
             h->g_factor[0].reset();
             h->g_solve.clear();
         }
         if (!h->d_f32)
         {
             HYB_CUDA(cudaMalloc(&h->d_f32, slab * sizeof(float)));
+            HYB_CUDA(cudaMalloc(&h->d_w32, std::max<int64_t>(1, S.w_elems) * sizeof(float)));
             if (S.n_inv > 0)
                 HYB_CUDA(cudaMalloc(&h->d_dinv, (size_t)S.n_inv * 4096 * sizeof(float)));
             h->g_factor[1].reset();
@@ -2642,7 +2699,7 @@ HYB_API int hyb_solve(hyb_system *h, const double *b, double *x, uint64_t nrhs, 
         // the plain drop-in solve: one substitution with the FP64 factors
         HYB_CUDA(cudaMemcpyAsync(h->d_x, h->d_b, bytes, cudaMemcpyDeviceToDevice, h->stream));
         auto &slot = h->g_solve[{HYB_PRECISION_FP64, nr}];
-        rc = substitute<double, double>(h, h->d_f64, h->d_x, h->d_scr64, nr, slot);
+        rc = substitute<double>(h, h->d_f64, h->d_x, h->d_scr64, nr, slot);
         if (rc != HYB_SUCCESS)
             return rc;
         if (want_residual)
@@ -3282,7 +3339,7 @@ extern "C" HYB_API int hyb_solve_fp64_noalloc(hyb_system *h, const double *b, do
     if (x != b)
         HYB_CUDA(cudaMemcpyAsync(x, b, len, cudaMemcpyDeviceToDevice, h->stream));
     uint64_t launches = 0;
-    rc = enqueue_solve<double, double>(h, h->d_f64, x, scratch, (int)nrhs, launches);
+    rc = enqueue_solve<double>(h, h->d_f64, x, scratch, (int)nrhs, launches);
     if (rc != HYB_SUCCESS)
         return rc;
     HYB_CUDA(cudaStreamSynchronize(h->stream));

@@ -13,6 +13,15 @@ namespace hyb
 // slab, so every block starts 256-byte aligned in FP64 and 128-byte aligned in FP32.
 constexpr int64_t kBlockAlign = 32;
 
+// Solve (hyb_solve.cuh): early blocks of a pivot's row per item, late blocks of it, and the rows of the
+// pivots that keep W = D^{-1} L for the late blocks. Smaller pivots substitute in less time than
+// the product with W would save; larger ones do not fit k_late.
+constexpr int kFlowGroup = 8;
+constexpr int kFlowLate = 2;
+constexpr int kFlowLateMin = 16;
+constexpr int kFlowLateMax = 128;
+constexpr int kFlowPad = 32; // elements a W block is padded to
+
 // Result of the symbolic phase: the reference's elimination replayed on the block
 // pattern alone. Everything the device schedule needs is precomputed here.
 struct Symbolic
@@ -52,13 +61,18 @@ struct Symbolic
     std::vector<int64_t> upd2_pref; // [n+1] prefix of ceil(|lower column| / 2) * |upper row| (row pairs)
     std::vector<int64_t> split_pref; // [n+1] prefix of n_lc + n_up: blocks whose BF16 split a tensor-core level stages
     std::vector<int64_t> tc_pref;    // [n+1] prefix of n_lc * ceil(n_up / 2): tensor-core update tiles
-    std::vector<int64_t> fwd_pref;  // [n+1] prefix of lower-row block counts
-    std::vector<int64_t> fwdu_pref; // [n+1] prefix of max(1, lower-row block count): forward solve units
-    std::vector<int32_t> fwd_item_p; // [fwdu_pref[n]] pivot slot of each forward dataflow item
-    std::vector<int32_t> bwd_item_p; // backward dataflow items (levels descending, max(1, n_up) per pivot)
+    std::vector<int64_t> fwdu_pref; // [n+1] prefix of forward solve items (early groups + the late item)
+    std::vector<int32_t> fwd_item_p; // [fwdu_pref[n]] pivot slot of each forward item
+    std::vector<int32_t> bwd_item_p; // backward items (levels descending)
     std::vector<int64_t> bwd_first;  // [n] first backward item of each pivot slot
-    std::vector<int64_t> fwd_rows;  // [n+1] prefix of lower-row block count * pivot size, padded to 4 (scratch rows)
-    std::vector<int64_t> bwd_rows;  // [n+1] prefix of upper-row block count * pivot size, padded to 4
+    std::vector<int64_t> bwd_lvl;    // [L+1] first backward item of level l (levels descending), [L]: unused
+    std::vector<int64_t> fwd_rows;  // [n+1] prefix of items * pivot size, padded to 4 (scratch rows)
+    std::vector<int64_t> bwd_rows;  // [n+1] the same, backward
+    std::vector<int64_t> w_off;     // [n] offset of a row's W blocks, one after the other, -1 where it has none
+    std::vector<int32_t> w_row, w_blk; // per W block: block row, filled index of the lower block
+    std::vector<int64_t> w_out;     // per W block: its offset
+    int64_t w_elems = 0;            // scalars of all W blocks (padded)
+    int32_t w_cols = 0;             // widest W block
     std::vector<int32_t> inv_idx;   // [n] slot of a 64-row block row's FP32 diagonal inverse (-1: other sizes)
     std::vector<int32_t> inv_row;   // [n_inv] block row of each inverse slot
     int64_t n_inv = 0;              // block rows of 64
@@ -135,8 +149,8 @@ struct Symbolic
 
     int64_t max_split_blocks = 0;    // max over uniform-64 levels of the split_pref span
     int64_t max_tc_targets = 0;       // max over uniform-64 levels of the upd_pref span (target table)
-    int64_t max_fwd_scratch_rows = 0; // max over levels of fwd_rows span
-    int64_t max_bwd_scratch_rows = 0;
+    int64_t max_fwd_scratch_rows = 0; // max over levels of lower (upper) blocks * pivot size, padded: at least
+    int64_t max_bwd_scratch_rows = 0; // the fwd_rows (bwd_rows) span; the limit of hyb_solve_fp64_noalloc
     double factor_flops = 0;          // exact algorithmic flops of the factorization
     int64_t factor_values = 0;        // unpadded scalars in the filled pattern
 

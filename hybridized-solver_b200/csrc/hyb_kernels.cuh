@@ -39,13 +39,16 @@ struct DevSym
     const int64_t *upd2_pref;
     const int64_t *split_pref;
     const int64_t *tc_pref;
-    const int64_t *fwd_pref;
     const int64_t *fwdu_pref;
-    const int32_t *fwd_item_p; // dataflow forward solve: pivot slot of item j (fwdu_pref order)
-    const int32_t *bwd_item_p; // dataflow backward solve: pivot slot of item j (levels descending)
+    const int32_t *fwd_item_p; // forward solve: pivot slot of item j (fwdu_pref order)
+    const int32_t *bwd_item_p; // backward solve: pivot slot of item j (levels descending)
     const int64_t *bwd_first;  // [n] first backward item of pivot slot p
     const int64_t *fwd_rows;
     const int64_t *bwd_rows;
+    const int64_t *w_off; // [n] offset of a row's W blocks (Symbolic::w_off), -1: none
+    const int32_t *w_row; // [W blocks] block row, filled index of the lower block and offset of each
+    const int32_t *w_blk;
+    const int64_t *w_out;
     const int32_t *inv_idx; // [n] slot of a 64-row block row's FP32 diagonal inverse (-1: none)
     const int32_t *inv_row; // [n_inv] block row of each inverse slot
     const int32_t *mt_tgt;
@@ -1554,47 +1557,9 @@ __global__ void __launch_bounds__(kThreads) k_update_listed(DevSym S, T *__restr
 // ----------------------------------------------------------------------------------
 // Solve. Vectors are dof x nrhs row-major in type V.
 //
-// Partial products of one block against the vector: out[i][r] = sum_q blk[i][q] * y[q][r]
-// for an m x K block; one warp per output row.
-// out = B y for one m x K block B (row-major) of the factors: every row is split over a
-// group of tpr consecutive threads (the largest power of two, at most 32, with 2 tpr m >
-// blockDim), each summing every tpr-th column, so all of the CTA's loads are in flight at
-// once; the group's sums are combined by an xor butterfly. With kL2, y is read from L2.
-template <bool kL2 = false, typename T, typename V>
-__device__ __forceinline__ void block_gemv(const T *__restrict__ blk, int m, int K, const V *y, V *__restrict__ out,
-                                           int nrhs)
-{
-    const int nt = blockDim.x;
-    int tpr = 1;
-    while (tpr < 32 && 2 * tpr * m <= nt)
-        tpr *= 2;
-    const int q = threadIdx.x & (tpr - 1), rl = threadIdx.x / tpr, rows = nt / tpr;
-    for (int r0 = 0; r0 < m; r0 += rows)
-    {
-        const int i = r0 + rl;
-        for (int r = 0; r < nrhs; ++r)
-        {
-            V s = 0;
-            if (i < m)
-            {
-                const T *row = blk + (int64_t)i * K;
-#pragma unroll 8
-                for (int c = q; c < K; c += tpr)
-                    s += (V)row[c] * (kL2 ? __ldcg(y + (int64_t)c * nrhs + r) : y[(int64_t)c * nrhs + r]);
-            }
-            for (int o = tpr >> 1; o > 0; o >>= 1)
-                s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (q == 0 && i < m)
-                out[(int64_t)i * nrhs + r] = s;
-        }
-    }
-}
-
-// One launch per stage and direction. Every CTA of a pivot forms one partial product (a
-// block of the pivot's lower row, forward, or upper row, backward, against the vector),
-// publishes it and takes a ticket; the CTA that takes the pivot's last ticket finishes the
-// pivot -- sums the partials in ascending block order and, forward, applies D^{-1}. No CTA
-// waits for another, so nothing can stall; the ticket is reset for the next solve.
+// In the staged forms every CTA of a pivot publishes its partial sums and takes a ticket; the CTA
+// that takes the pivot's last ticket finishes the pivot. No CTA waits for another, so nothing
+// can stall; the ticket is reset for the next solve.
 // Returns true in the CTA that must finish pivot p.
 __device__ __forceinline__ bool last_ticket(int *tickets, int64_t p, int64_t nparts)
 {
@@ -1936,42 +1901,6 @@ template <typename V> __device__ void sum_partials(const V *part, int64_t nparts
     }
 }
 
-// out[e] = (y[e] - early[e]) - late[e], either term absent when null; early is read from
-// L2, late from L2 when late_l2 (written by another CTA) and directly otherwise.
-template <typename V>
-__device__ __forceinline__ void combine_partials(V *out, const V *y, const V *early, const V *late, bool late_l2,
-                                                 int E)
-{
-    for (int e = threadIdx.x; e < E; e += blockDim.x)
-    {
-        V v = y[e];
-        if (early)
-            v -= __ldcg(early + e);
-        if (late)
-            v -= late_l2 ? __ldcg(late + e) : late[e];
-        out[e] = v;
-    }
-}
-
-
-// The first kStageRegs x blockDim values of a diagonal block, loaded into registers
-// early so their latency overlaps other work before they go to shared memory.
-constexpr int kStageRegs = 16;
-template <typename T> struct DiagRegs
-{
-    T v[kStageRegs];
-};
-
-template <typename T> __device__ __forceinline__ void diag_load(DiagRegs<T> &dv, const T *gd, int mm)
-{
-#pragma unroll
-    for (int q = 0; q < kStageRegs; ++q)
-    {
-        const int i = q * (int)blockDim.x + (int)threadIdx.x;
-        dv.v[q] = i < mm ? gd[i] : T(0);
-    }
-}
-
 // Explicit inverses of the 64x64 diagonal blocks for the FP32 solves inside the mixed
 // form's refinement, where the inner solve only has to be a good approximation (the FP64
 // residual decides convergence): X = D^{-1} from D's LU factors, column j of X by thread
@@ -2015,437 +1944,14 @@ __global__ void __launch_bounds__(kInvThreads) k_diag_inv64(DevSym S, const T *_
         xt[i] = y[i];
 }
 
-// The registers a forward finisher fills for pivot k before it waits: k's inverse when
-// the factorization built one (dinv set), else D_k when it will be staged.
-template <typename T>
-__device__ __forceinline__ void fwd_preload(DiagRegs<T> &dv, const DevSym &S, const T *__restrict__ slab,
-                                            const T *__restrict__ dinv, int64_t k, int stage_diag)
-{
-    if (dinv && S.inv_idx[k] >= 0)
-        diag_load(dv, dinv + (int64_t)S.inv_idx[k] * 4096, 4096);
-    else if (stage_diag)
-        diag_load(dv, slab + S.blk_off[S.diag_pos[k]], S.size[k] * S.size[k]);
-}
-
-// y_k <- D_k^{-1} acc for pivot k (acc: m x nrhs in shared memory). With an inverse (dinv
-// set, 64-row pivot): a product with the inverse held in `dv` -- thread t has
-// X(t mod 64, 4q + t / 64), q < 16 -- its four partial sums per row added in a fixed
-// order. Otherwise substitution with the LU factors, D_k staged in shared memory with an
-// odd row stride (column reads of the substitution hit distinct banks) when stage_diag,
-// from the registers `dv` filled by diag_load.
-template <typename T, typename V>
-__device__ void fwd_solve_store(const DevSym &S, const T *__restrict__ slab, const T *__restrict__ dinv,
-                                V *__restrict__ yk, int64_t k, int nrhs, int stage_diag, unsigned char *smem_raw,
-                                V *acc, const DiagRegs<T> &dv)
-{
-    const int m = S.size[k];
-    static_assert(kStageRegs * kThreads == 64 * 64, "one 64x64 inverse fills the finisher's registers");
-    if (dinv && S.inv_idx[k] >= 0)
-    {
-        __shared__ V s_part[kThreads];
-        const int tid = threadIdx.x, g = tid >> 6;
-        __syncthreads(); // acc is complete
-        for (int c = 0; c < nrhs; ++c)
-        {
-            V s = V(0);
-#pragma unroll
-            for (int q = 0; q < kStageRegs; ++q)
-                s += (V)dv.v[q] * acc[(4 * q + g) * nrhs + c];
-            s_part[tid] = s;
-            __syncthreads();
-            if (tid < 64)
-                yk[tid * nrhs + c] = (s_part[tid] + s_part[64 + tid]) + (s_part[128 + tid] + s_part[192 + tid]);
-            __syncthreads();
-        }
-        return;
-    }
-    const T *gd = slab + S.blk_off[S.diag_pos[k]];
-    const int mm = m * m, nt = blockDim.x, tid = threadIdx.x;
-    const T *d = gd;
-    int ldd = m;
-    const size_t acc_bytes = ((size_t)m * nrhs * sizeof(V) + 15) / 16 * 16;
-    if (stage_diag)
-    {
-        T *sd = reinterpret_cast<T *>(smem_raw + acc_bytes);
-        ldd = m | 1;
-        if ((m & (m - 1)) == 0)
-        {
-            const int sh = __ffs(m) - 1;
-#pragma unroll
-            for (int q = 0; q < kStageRegs; ++q)
-            {
-                const int i = q * nt + tid;
-                if (i < mm)
-                    sd[(i >> sh) * ldd + (i & (m - 1))] = dv.v[q];
-            }
-        }
-        else
-        {
-#pragma unroll
-            for (int q = 0; q < kStageRegs; ++q)
-            {
-                const int i = q * nt + tid;
-                if (i < mm)
-                    sd[(i / m) * ldd + i % m] = dv.v[q];
-            }
-        }
-        for (int i = kStageRegs * nt + tid; i < mm; i += nt)
-            sd[(i / m) * ldd + i % m] = gd[i];
-        d = sd;
-    }
-    __syncthreads();
-    // unit lower, then upper; one warp per right-hand side
-    const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int r = warp; r < nrhs; r += nw)
-    {
-        if (m <= 32)
-            warp_lu_solve<1>(d, ldd, m, acc, r, nrhs);
-        else if (m <= 64)
-            warp_lu_solve<2>(d, ldd, m, acc, r, nrhs);
-        else if (m <= 96)
-            warp_lu_solve1<3>(d, ldd, m, acc, r, nrhs);
-        else if (m <= 128)
-            warp_lu_solve1<4>(d, ldd, m, acc, r, nrhs);
-        else
-            warp_lu_solve_smem(d, ldd, m, acc, r, nrhs);
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < m * nrhs; i += blockDim.x)
-        yk[i] = acc[i];
-}
-
-// Partials of a pivot with n blocks: the "late" block -- the one whose source is final last,
-// the last lower block (forward) or the first upper block (backward) -- and the n - 1 early
-// ones, contiguous. Both substitution forms compute y - (sum of the early partials, in
-// sum_partials' order) - late partial, so they agree bit for bit.
-// Forward stage: y_k <- D_k^{-1} (y_k - sum_s L(k,s) y_s) for the stage's pivots
-// (block_system_apply_operations, src/blocks.c:729-769). Units: fwdu_pref, one per lower
-// block of a pivot (at least one per pivot).
-template <typename T, typename V>
-__global__ void __launch_bounds__(kThreads, 1)
-    k_fwd_stage(DevSym S, const T *__restrict__ slab, V *__restrict__ y, V *__restrict__ scratch,
-                int *__restrict__ tickets, int64_t p0, int64_t p1, int nrhs, int stage_diag,
-                const T *__restrict__ dinv)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int64_t u = S.fwdu_pref[p0] + blockIdx.x;
-    const int64_t p = find_owner(S.fwdu_pref, p0, p1, u);
-    const int64_t k = S.piv[p];
-    const int m = S.size[k];
-    const int64_t nparts = S.diag_pos[k] - S.row_ptr[k];
-    V *part = scratch + (S.fwd_rows[p] - S.fwd_rows[p0]) * nrhs;
-    const int E = m * nrhs;
-    if (nparts > 0)
-    {
-        const int64_t j = u - S.fwdu_pref[p];
-        const int64_t blk = S.row_ptr[k] + j;
-        const int32_t src = S.cols[blk];
-        block_gemv(slab + S.blk_off[blk], m, S.size[src], y + S.dof_off[src] * nrhs, part + j * E, nrhs);
-        if (!last_ticket(tickets, p, nparts))
-            return;
-    }
-    __shared__ __align__(16) V red[kThreads * 16 / sizeof(V)];
-    DiagRegs<T> dv;
-    fwd_preload(dv, S, slab, dinv, k, stage_diag);
-    if (nparts > 1)
-    {
-        sum_partials(part, nparts - 1, E, part, red);
-        __syncthreads();
-    }
-    V *acc = reinterpret_cast<V *>(smem_raw);
-    V *yk = y + S.dof_off[k] * nrhs;
-    combine_partials(acc, yk, nparts > 1 ? part : nullptr, nparts > 0 ? part + (nparts - 1) * E : nullptr, true, E);
-    fwd_solve_store(S, slab, dinv, yk, k, nrhs, stage_diag, smem_raw, acc, dv);
-}
-
-// Backward stage: y_k -= sum_c U(k,c) y_c over the upper blocks of the stage's pivots
-// (block_system_solve_u, src/blocks.c:771-800). Units: trsm_pref, one per upper block.
-template <typename T, typename V>
-__global__ void __launch_bounds__(kThreads, 2)
-    k_bwd_stage(DevSym S, const T *__restrict__ slab, V *__restrict__ y, V *__restrict__ scratch,
-                int *__restrict__ tickets, int64_t p0, int64_t p1, int nrhs)
-{
-    const int64_t u = S.trsm_pref[p0] + blockIdx.x;
-    const int64_t p = find_owner(S.trsm_pref, p0, p1, u);
-    const int64_t k = S.piv[p];
-    const int m = S.size[k];
-    const int64_t nparts = S.row_ptr[k + 1] - S.diag_pos[k] - 1;
-    const int64_t j = u - S.trsm_pref[p];
-    const int64_t blk = S.diag_pos[k] + 1 + j;
-    const int32_t c = S.cols[blk];
-    V *part = scratch + (S.bwd_rows[p] - S.bwd_rows[p0]) * nrhs;
-    const int E = m * nrhs;
-    block_gemv(slab + S.blk_off[blk], m, S.size[c], y + S.dof_off[c] * nrhs, part + j * E, nrhs);
-    if (!last_ticket(tickets, p, nparts))
-        return;
-    __shared__ __align__(16) V red[kThreads * 16 / sizeof(V)];
-    if (nparts > 1)
-    {
-        sum_partials(part + E, nparts - 1, E, part + E, red);
-        __syncthreads();
-    }
-    V *yk = y + S.dof_off[k] * nrhs;
-    combine_partials(yk, yk, nparts > 1 ? part + E : nullptr, part, true, E);
-}
-
-// ----------------------------------------------------------------------------------
-// Dataflow substitution: one cooperative launch per direction instead of one launch per
-// level. A work item is one partial product -- block (k, s) of a pivot's lower row
-// (forward) or (k, c) of its upper row (backward) against the source's final vector --
-// and pivots without such blocks get one empty item. Items are ordered by level (forward
-// ascending, backward descending) and CTA b takes items b, b + G, ... in order. Before its
-// product an item waits until the source block row's flag carries this solve's tag; the
-// CTA that takes a pivot's last ticket finishes it and sets the pivot's flag. Every wait
-// depends only on items earlier in the order and all CTAs are resident (cooperative
-// launch), so the waits end; each is also bounded in time (wait_ns; ST_TIMEOUT in
-// `status`, after which every wait returns at once). Source vectors are read from L2 (__ldcg): another
-// SM may have written them after this SM cached a neighbouring line.
-__device__ __forceinline__ int ld_acquire(const int *p)
-{
-    int v;
-    asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ void st_release(int *p, int v)
-{
-    asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-// Waits (thread 0, at most wait_ns) until *flag == tag; CTA-uniform result.
-__device__ __forceinline__ bool wait_flag(const int *flag, int tag, int *status, uint64_t wait_ns)
-{
-    __shared__ int s_ok;
-    if (threadIdx.x == 0)
-    {
-        int ok = 1;
-        if (ld_acquire(flag) != tag)
-        {
-            const uint64_t t0 = global_ns();
-            while (ld_acquire(flag) != tag)
-            {
-                if (schedule_aborted(status) || global_ns() - t0 > wait_ns)
-                {
-                    atomicOr(status + ST_TIMEOUT, 1);
-                    ok = 0;
-                    break;
-                }
-                __nanosleep(64);
-            }
-        }
-        s_ok = ok;
-    }
-    __syncthreads();
-    const bool ok = s_ok != 0;
-    __syncthreads(); // s_ok is reused by the next wait
-    return ok;
-}
-
-// Marks block row k final for this solve (after every thread's writes of y_k).
-__device__ __forceinline__ void publish_flag(int *flag, int tag)
-{
-    __syncthreads();
-    if (threadIdx.x == 0)
-    {
-        __threadfence();
-        st_release(flag, tag);
-    }
-}
-
-
-// A block's share of the row-group product (block_gemv's mapping) held in registers, so
-// it can be loaded before the wait for the vector it multiplies. Used when one pass covers
-// the block and a thread's share fits (kGemvRegs values); otherwise `ok` is false.
-constexpr int kGemvRegs = 16;
-template <typename T> struct GemvRegs
-{
-    T v[kGemvRegs];
-    bool ok;
-};
-
+// Threads per row of a product with an m-row block: the largest power of two, at most 32, that leaves a CTA's
+// threads at least m rows.
 template <typename T> __device__ __forceinline__ int gemv_tpr(int m)
 {
     int tpr = 1;
     while (tpr < 32 && 2 * tpr * m <= (int)blockDim.x)
         tpr *= 2;
     return tpr;
-}
-
-template <typename T> __device__ __forceinline__ void gemv_load(GemvRegs<T> &g, const T *__restrict__ blk, int m, int K)
-{
-    const int tpr = gemv_tpr<T>(m), rows = blockDim.x / tpr;
-    const int q = threadIdx.x & (tpr - 1), i = threadIdx.x / tpr;
-    g.ok = rows >= m && (K + tpr - 1) / tpr <= kGemvRegs;
-    if (!g.ok)
-        return;
-#pragma unroll
-    for (int c = 0; c < kGemvRegs; ++c)
-    {
-        const int col = q + c * tpr;
-        g.v[c] = (i < m && col < K) ? blk[(int64_t)i * K + col] : T(0);
-    }
-}
-
-// out = B y with B's share in registers; the same products and order as block_gemv<true>.
-template <typename T, typename V>
-__device__ __forceinline__ void gemv_finish(const GemvRegs<T> &g, int m, int K, const V *y, V *__restrict__ out,
-                                            int nrhs)
-{
-    const int tpr = gemv_tpr<T>(m);
-    const int q = threadIdx.x & (tpr - 1), i = threadIdx.x / tpr;
-    for (int r = 0; r < nrhs; ++r)
-    {
-        V s = 0;
-        if (i < m)
-        {
-#pragma unroll
-            for (int c = 0; c < kGemvRegs; ++c)
-            {
-                const int col = q + c * tpr;
-                if (col < K)
-                    s += (V)g.v[c] * __ldcg(y + (int64_t)col * nrhs + r);
-            }
-        }
-        for (int o = tpr >> 1; o > 0; o >>= 1)
-            s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (q == 0 && i < m)
-            out[(int64_t)i * nrhs + r] = s;
-    }
-}
-
-// Pulls a block into L2 ahead of its use (one 128-byte line per thread and step).
-template <typename T> __device__ __forceinline__ void prefetch_l2(const T *p, int64_t elems)
-{
-    const char *c = reinterpret_cast<const char *>(p);
-    const int64_t bytes = elems * (int64_t)sizeof(T);
-    for (int64_t off = (int64_t)threadIdx.x * 128; off < bytes; off += (int64_t)blockDim.x * 128)
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(c + off));
-}
-
-// Forward direction; partials of pivot slot p at scratch + fwd_rows[p] * nrhs. The late
-// item (the pivot's last lower block, whose source is the most recent pivot) finishes the
-// pivot: it loads its diagonal block before waiting, keeps its own partial in shared
-// memory, and waits only for the pre-sum of the early partials, which the CTA taking the
-// last early ticket forms and flags in pflags.
-template <typename T, typename V>
-__global__ void __launch_bounds__(kThreads, 1)
-    k_fwd_flow(DevSym S, const T *__restrict__ slab, V *__restrict__ y, V *__restrict__ scratch,
-               int *__restrict__ tickets, int *__restrict__ flags, int *__restrict__ pflags, int tag, int64_t n_items,
-               int nrhs, int stage_diag, const T *__restrict__ dinv, int *status, uint64_t wait_ns)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ __align__(16) V red[kThreads * 16 / sizeof(V)];
-    V *acc = reinterpret_cast<V *>(smem_raw); // m * nrhs
-    for (int64_t j = blockIdx.x; j < n_items; j += gridDim.x)
-    {
-        const int64_t p = S.fwd_item_p[j];
-        const int64_t k = S.piv[p];
-        const int m = S.size[k];
-        const int E = m * nrhs;
-        const int64_t nparts = S.diag_pos[k] - S.row_ptr[k];
-        V *part = scratch + S.fwd_rows[p] * nrhs;
-        V *yk = y + S.dof_off[k] * nrhs;
-        const T *gd = slab + S.blk_off[S.diag_pos[k]];
-        DiagRegs<T> dv;
-        if (nparts == 0)
-        {
-            fwd_preload(dv, S, slab, dinv, k, stage_diag);
-            combine_partials(acc, yk, (const V *)nullptr, (const V *)nullptr, false, E);
-            fwd_solve_store(S, slab, dinv, yk, k, nrhs, stage_diag, smem_raw, acc, dv);
-            publish_flag(flags + k, tag);
-            continue;
-        }
-        const int64_t local = j - S.fwdu_pref[p];
-        const bool late = local == nparts - 1;
-        const int64_t blk = S.row_ptr[k] + local;
-        const int32_t src = S.cols[blk];
-        const int K = S.size[src];
-        const bool inv = dinv && S.inv_idx[k] >= 0;
-        if (local == 0 && !late && (stage_diag || inv)) // the finisher will load D_k or its inverse: into L2 now
-            prefetch_l2(inv ? dinv + (int64_t)S.inv_idx[k] * 4096 : gd, inv ? (int64_t)4096 : (int64_t)m * m);
-        if (late)
-            fwd_preload(dv, S, slab, dinv, k, stage_diag);
-        GemvRegs<T> g;
-        gemv_load(g, slab + S.blk_off[blk], m, K);
-        if (!wait_flag(flags + src, tag, status, wait_ns))
-            return;
-        V *dst = late ? acc : part + local * E;
-        if (g.ok)
-            gemv_finish(g, m, K, y + S.dof_off[src] * nrhs, dst, nrhs);
-        else
-            block_gemv<true>(slab + S.blk_off[blk], m, K, y + S.dof_off[src] * nrhs, dst, nrhs);
-        if (!late)
-        {
-            if (!last_ticket(tickets, p, nparts - 1))
-                continue;
-            sum_partials(part, nparts - 1, E, part, red);
-            publish_flag(pflags + p, tag);
-            continue;
-        }
-        if (nparts > 1 && !wait_flag(pflags + p, tag, status, wait_ns))
-            return;
-        __syncthreads(); // the late partial is in acc
-        combine_partials(acc, yk, nparts > 1 ? (const V *)part : nullptr, (const V *)acc, false, E);
-        fwd_solve_store(S, slab, dinv, yk, k, nrhs, stage_diag, smem_raw, acc, dv);
-        publish_flag(flags + k, tag);
-    }
-}
-
-// Backward direction; partials of pivot slot p at scratch + bwd_rows[p] * nrhs. Item q of a
-// pivot with n upper blocks takes block (q + 1) mod n, so the late block 0 (its source is
-// the most recently finished pivot) comes last and finishes the pivot as in k_fwd_flow.
-template <typename T, typename V>
-__global__ void __launch_bounds__(kThreads, 2)
-    k_bwd_flow(DevSym S, const T *__restrict__ slab, V *__restrict__ y, V *__restrict__ scratch,
-               int *__restrict__ tickets, int *__restrict__ flags, int *__restrict__ pflags, int tag, int64_t n_items,
-               int nrhs, int *status, uint64_t wait_ns)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ __align__(16) V red[kThreads * 16 / sizeof(V)];
-    V *acc = reinterpret_cast<V *>(smem_raw); // m * nrhs
-    for (int64_t j = blockIdx.x; j < n_items; j += gridDim.x)
-    {
-        const int64_t p = S.bwd_item_p[j];
-        const int64_t k = S.piv[p];
-        const int m = S.size[k];
-        const int E = m * nrhs;
-        const int64_t nparts = S.row_ptr[k + 1] - S.diag_pos[k] - 1;
-        if (nparts == 0)
-        {
-            publish_flag(flags + k, tag);
-            continue;
-        }
-        const int64_t q = j - S.bwd_first[p];
-        const int64_t b = (q + 1) % nparts;
-        const bool late = b == 0;
-        const int64_t blk = S.diag_pos[k] + 1 + b;
-        const int32_t c = S.cols[blk];
-        const int K = S.size[c];
-        V *part = scratch + S.bwd_rows[p] * nrhs;
-        GemvRegs<T> g;
-        gemv_load(g, slab + S.blk_off[blk], m, K);
-        if (!wait_flag(flags + c, tag, status, wait_ns))
-            return;
-        V *dst = late ? acc : part + b * E;
-        if (g.ok)
-            gemv_finish(g, m, K, y + S.dof_off[c] * nrhs, dst, nrhs);
-        else
-            block_gemv<true>(slab + S.blk_off[blk], m, K, y + S.dof_off[c] * nrhs, dst, nrhs);
-        if (!late)
-        {
-            if (!last_ticket(tickets, p, nparts - 1))
-                continue;
-            sum_partials(part + E, nparts - 1, E, part + E, red);
-            publish_flag(pflags + p, tag);
-            continue;
-        }
-        if (nparts > 1 && !wait_flag(pflags + p, tag, status, wait_ns))
-            return;
-        __syncthreads(); // the late partial is in acc
-        V *yk = y + S.dof_off[k] * nrhs;
-        combine_partials(yk, yk, nparts > 1 ? (const V *)(part + E) : nullptr, (const V *)acc, false, E);
-        publish_flag(flags + k, tag);
-    }
 }
 
 // ----------------------------------------------------------------------------------

@@ -344,7 +344,6 @@ int symbolic_build(int64_t n, const uint64_t *sizes, const uint64_t *row_ptr, co
     S.upd2_pref.assign(n + 1, 0);
     S.split_pref.assign(n + 1, 0);
     S.tc_pref.assign(n + 1, 0);
-    S.fwd_pref.assign(n + 1, 0);
     S.fwdu_pref.assign(n + 1, 0);
     S.fwd_rows.assign(n + 1, 0);
     S.bwd_rows.assign(n + 1, 0);
@@ -357,6 +356,8 @@ int symbolic_build(int64_t n, const uint64_t *sizes, const uint64_t *row_ptr, co
             S.inv_row.push_back((int32_t)k);
         }
     S.n_inv = (int64_t)S.inv_row.size();
+    S.w_off.assign(n, -1);
+    std::vector<int64_t> fwd_span(n + 1, 0), bwd_span(n + 1, 0);
     double flops = 0;
     std::vector<double> piv_upd_flops(n), piv_upd_c(n), piv_upd_ab(n);
     for (int64_t p = 0; p < n; ++p)
@@ -372,12 +373,30 @@ int symbolic_build(int64_t n, const uint64_t *sizes, const uint64_t *row_ptr, co
         S.upd2_pref[p + 1] = S.upd2_pref[p] + (n_lc + 1) / 2 * n_up;
         S.split_pref[p + 1] = S.split_pref[p] + n_lc + n_up;
         S.tc_pref[p + 1] = S.tc_pref[p] + n_lc * ((n_up + 1) / 2);
-        S.fwd_pref[p + 1] = S.fwd_pref[p] + n_lr;
-        S.fwdu_pref[p + 1] = S.fwdu_pref[p] + std::max<int64_t>(1, n_lr);
+        // solve items: the early blocks of the row in groups, then one item for the late ones
+        const bool has_w = n_lr > 0 && S.size[k] >= kFlowLateMin && S.size[k] <= kFlowLateMax;
+        const int64_t ne = n_lr - std::min<int64_t>(n_lr, has_w ? kFlowLate : 1);
+        const int64_t nf = (ne + kFlowGroup - 1) / kFlowGroup + 1;
+        const int64_t nb = (std::max<int64_t>(0, n_up - kFlowLate) + kFlowGroup - 1) / kFlowGroup + 1;
+        S.fwdu_pref[p + 1] = S.fwdu_pref[p] + nf;
         // partial-product spans padded to 4 values, so every pivot's partials start on a
         // 16-byte boundary in the staged (per-stage) and the dataflow (global) layouts alike
-        S.fwd_rows[p + 1] = S.fwd_rows[p] + (n_lr * S.size[k] + 3) / 4 * 4;
-        S.bwd_rows[p + 1] = S.bwd_rows[p] + (n_up * S.size[k] + 3) / 4 * 4;
+        S.fwd_rows[p + 1] = S.fwd_rows[p] + ((n_lr > 0 ? nf : 0) * S.size[k] + 3) / 4 * 4;
+        S.bwd_rows[p + 1] = S.bwd_rows[p] + ((n_up > 0 ? nb : 0) * S.size[k] + 3) / 4 * 4;
+        fwd_span[p + 1] = fwd_span[p] + (n_lr * S.size[k] + 3) / 4 * 4;
+        bwd_span[p + 1] = bwd_span[p] + (n_up * S.size[k] + 3) / 4 * 4;
+        if (has_w)
+        {
+            S.w_off[k] = S.w_elems;
+            for (int64_t j = S.row_ptr[k] + ne; j < S.diag_pos[k]; ++j)
+            {
+                S.w_row.push_back((int32_t)k);
+                S.w_blk.push_back((int32_t)j);
+                S.w_out.push_back(S.w_elems);
+                S.w_elems += round_up((int64_t)S.size[k] * S.size[S.cols[j]], kFlowPad);
+                S.w_cols = std::max(S.w_cols, S.size[S.cols[j]]);
+            }
+        }
         double up_cols = 0, lc_rows = 0;
         for (int64_t j = S.diag_pos[k] + 1; j < S.row_ptr[k + 1]; ++j)
             up_cols += S.size[S.cols[j]];
@@ -396,17 +415,21 @@ int symbolic_build(int64_t n, const uint64_t *sizes, const uint64_t *row_ptr, co
         for (int64_t j = S.fwdu_pref[p]; j < S.fwdu_pref[p + 1]; ++j)
             S.fwd_item_p[j] = (int32_t)p;
     S.bwd_item_p.clear();
-    S.bwd_item_p.reserve(S.trsm_pref[n] + n);
     S.bwd_first.assign(n, 0);
+    S.bwd_lvl.assign(S.n_levels + 1, 0);
     for (int64_t l = S.n_levels - 1; l >= 0; --l)
+    {
+        S.bwd_lvl[l] = (int64_t)S.bwd_item_p.size();
         for (int64_t p = S.lvl_ptr[l]; p < S.lvl_ptr[l + 1]; ++p)
         {
             const int64_t k = S.piv[p];
             const int64_t n_up = S.row_ptr[k + 1] - S.diag_pos[k] - 1;
             S.bwd_first[p] = (int64_t)S.bwd_item_p.size();
-            for (int64_t j = 0; j < std::max<int64_t>(1, n_up); ++j)
+            const int64_t nb = (std::max<int64_t>(0, n_up - kFlowLate) + kFlowGroup - 1) / kFlowGroup + 1;
+            for (int64_t j = 0; j < nb; ++j)
                 S.bwd_item_p.push_back((int32_t)p);
         }
+    }
 
     // ---- Level shapes, scratch spans and listed (conflicting) update levels.
     S.shape.assign(S.n_levels, {});
@@ -463,9 +486,9 @@ int symbolic_build(int64_t n, const uint64_t *sizes, const uint64_t *row_ptr, co
             S.max_tc_targets = std::max(S.max_tc_targets, S.upd_pref[S.lvl_ptr[l + 1]] - S.upd_pref[S.lvl_ptr[l]]);
         }
         S.max_fwd_scratch_rows =
-            std::max(S.max_fwd_scratch_rows, S.fwd_rows[S.lvl_ptr[l + 1]] - S.fwd_rows[S.lvl_ptr[l]]);
+            std::max(S.max_fwd_scratch_rows, fwd_span[S.lvl_ptr[l + 1]] - fwd_span[S.lvl_ptr[l]]);
         S.max_bwd_scratch_rows =
-            std::max(S.max_bwd_scratch_rows, S.bwd_rows[S.lvl_ptr[l + 1]] - S.bwd_rows[S.lvl_ptr[l]]);
+            std::max(S.max_bwd_scratch_rows, bwd_span[S.lvl_ptr[l + 1]] - bwd_span[S.lvl_ptr[l]]);
         if (conflict)
         {
             S.lvl_listed[l] = 1;
