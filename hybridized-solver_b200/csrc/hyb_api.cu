@@ -409,6 +409,7 @@ int upload_symbolic(hyb_system *h)
         {S.fwdu_pref.data(), S.fwdu_pref.size() * 8, (const void **)&d.fwdu_pref},
         {S.fwd_item_p.data(), S.fwd_item_p.size() * 4, (const void **)&d.fwd_item_p},
         {S.bwd_item_p.data(), S.bwd_item_p.size() * 4, (const void **)&d.bwd_item_p},
+        {S.bwd_slot.data(), S.bwd_slot.size() * 4, (const void **)&d.bwd_slot},
         {S.bwd_first.data(), S.bwd_first.size() * 8, (const void **)&d.bwd_first},
         {S.fwd_rows.data(), S.fwd_rows.size() * 8, (const void **)&d.fwd_rows},
         {S.bwd_rows.data(), S.bwd_rows.size() * 8, (const void **)&d.bwd_rows},
@@ -740,42 +741,6 @@ int enqueue_pivots(hyb_system *h, T *slab, int64_t l, cudaStream_t st, uint64_t 
         HYB_LAUNCHED("k_trsm", l);
     }
     return enqueue_split<T>(h, slab, l, st, launches);
-}
-
-// Whether the pivot work of every level with 64-row pivots already wrote their FP32
-// inverses (the mixed form's inverse-and-products path, HYB_OPTION_ROW_PIVOTS 2).
-template <typename T> bool inverses_by_pivots(const hyb_system *h)
-{
-    const Symbolic &S = h->S;
-    const int mode64 = h->row_pivots < 0 ? (std::is_same_v<T, float> ? 2 : 0) : h->row_pivots;
-    if (!std::is_same_v<T, float> || mode64 != 2)
-        return false;
-    for (int64_t l = 0; l < S.n_levels; ++l)
-    {
-        bool has64 = false;
-        for (int64_t p = S.lvl_ptr[l]; p < S.lvl_ptr[l + 1] && !has64; ++p)
-            has64 = S.size[S.piv[p]] == 64;
-        if (has64 && !(fused_pivots(S.shape[l]) && S.shape[l].piv64 && tc_level<T>(h, l)))
-            return false;
-    }
-    return true;
-}
-
-// FP32 inverses of every 64-row diagonal block (mixed form), in one launch after the last
-// level. Only the solves read them; launched beside the stages instead, they slowed the
-// update CTAs that shared their SMs, and each level waits for its slowest update CTA.
-template <typename T> int enqueue_inverses(hyb_system *h, T *slab, uint64_t &launches)
-{
-    if constexpr (std::is_same_v<T, float>)
-    {
-        if (!h->d_dinv || h->S.n_inv == 0 || inverses_by_pivots<T>(h))
-            return HYB_SUCCESS;
-        hyb::k_diag_inv64<float>
-            <<<(unsigned)h->S.n_inv, hyb::kInvThreads, 0, h->stream>>>(h->ds, slab, h->d_dinv);
-        ++launches;
-        HYB_LAUNCHED("k_diag_inv64", h->S.n_levels - 1);
-    }
-    return HYB_SUCCESS;
 }
 
 template <typename T> T *&late_blocks(hyb_system *h);
@@ -1177,20 +1142,10 @@ template <typename T> int enqueue_factor(hyb_system *h, T *slab, uint64_t &launc
         HYB_CUDA(cudaEventRecord(h->ev_join, st2));
         HYB_CUDA(cudaStreamWaitEvent(st, h->ev_join, 0));
     }
-    if ((rc = enqueue_inverses<T>(h, slab, launches)) != HYB_SUCCESS ||
-        (rc = enqueue_late<T>(h, slab, launches)) != HYB_SUCCESS)
+    if ((rc = enqueue_late<T>(h, slab, launches)) != HYB_SUCCESS)
         return rc;
     HYB_CUDA(cudaGetLastError());
     return HYB_SUCCESS;
-}
-
-// The FP32 diagonal inverses a solve with factors of type T uses (mixed form only).
-template <typename T> const T *solve_dinv(const hyb_system *h)
-{
-    if constexpr (std::is_same_v<T, float>)
-        return h->d_dinv;
-    else
-        return nullptr;
 }
 
 // Largest diagonal block of the system.
@@ -1207,7 +1162,7 @@ int max_pivot(const Symbolic &S)
 template <typename T> int64_t solve_smem(const Symbolic &S, int nc, int &stage)
 {
     const int mp = max_pivot(S);
-    stage = hyb::flow_smem_bytes<T>(mp, nc, true) <= solve_smem_cap() ? 1 : 0;
+    stage = mp <= hyb::kFlowLateMax && hyb::flow_smem_bytes<T>(mp, nc, true) <= solve_smem_cap() ? 1 : 0;
     return hyb::flow_smem_bytes<T>(mp, nc, stage != 0);
 }
 
@@ -1218,7 +1173,7 @@ template <typename T, int NC>
 int enqueue_stages(hyb_system *h, const T *slab, T *y, T *scratch, int nrhs, uint64_t &launches)
 {
     const Symbolic &S = h->S;
-    const T *dinv = solve_dinv<T>(h), *wbuf = late_blocks<T>(h);
+    const T *wbuf = late_blocks<T>(h);
     cudaStream_t st = h->stream;
     int stage = 0;
     const int64_t smem = solve_smem<T>(S, NC, stage);
@@ -1229,19 +1184,20 @@ int enqueue_stages(hyb_system *h, const T *slab, T *y, T *scratch, int nrhs, uin
     HYB_CUDA(allow_smem(hyb::k_stage<T, NC, false>, (int)smem));
     for (int64_t l = 0; l < S.n_levels; ++l)
     {
-        const int64_t p0 = S.lvl_ptr[l], first = S.fwdu_pref[p0], units = S.fwdu_pref[S.lvl_ptr[l + 1]] - first;
-        hyb::k_stage<T, NC, true><<<(unsigned)units, hyb::kThreads, (size_t)smem, st>>>(
-            h->ds, slab, wbuf, y, scratch, h->d_tickets, dinv, first, S.fwd_rows[p0], nrhs, mp, stage);
+        const int64_t p0 = S.lvl_ptr[l], p1 = S.lvl_ptr[l + 1], first = S.fwdu_pref[p0];
+        const unsigned groups = (unsigned)(S.fwdu_pref[p1] - first);
+        hyb::k_stage<T, NC, true><<<groups + (unsigned)(p1 - p0), hyb::kFlowThreads, (size_t)smem, st>>>(
+            h->ds, slab, wbuf, y, scratch, h->d_tickets, p0, first, groups, nrhs, mp, stage);
         ++launches;
     }
     for (int64_t l = S.n_levels - 1; l >= 0; --l)
     {
-        const int64_t p0 = S.lvl_ptr[l], first = S.bwd_lvl[l];
-        const int64_t units = (l > 0 ? S.bwd_lvl[l - 1] : (int64_t)S.bwd_item_p.size()) - first;
-        if (S.trsm_pref[S.lvl_ptr[l + 1]] == S.trsm_pref[p0])
+        const int64_t p0 = S.lvl_ptr[l], p1 = S.lvl_ptr[l + 1], first = S.bwd_lvl[l];
+        const unsigned groups = (unsigned)((l > 0 ? S.bwd_lvl[l - 1] : (int64_t)S.bwd_item_p.size()) - first);
+        if (S.trsm_pref[p1] == S.trsm_pref[p0])
             continue; // no upper blocks
-        hyb::k_stage<T, NC, false><<<(unsigned)units, hyb::kThreads, (size_t)smem, st>>>(
-            h->ds, slab, wbuf, y, scratch, h->d_tickets, dinv, first, S.bwd_rows[p0], nrhs, mp, stage);
+        hyb::k_stage<T, NC, false><<<groups + (unsigned)(p1 - p0), hyb::kFlowThreads, (size_t)smem, st>>>(
+            h->ds, slab, wbuf, y, scratch, h->d_tickets, p0, first, groups, nrhs, mp, stage);
         ++launches;
     }
     HYB_CUDA(cudaGetLastError());
@@ -1278,21 +1234,27 @@ int launch_flow(hyb_system *h, const T *slab, T *y, hyb::Tagged<T> *scr, int tag
     if (smem > solve_smem_cap())
         return HYB_TOO_LARGE;
     HYB_CUDA(allow_smem(hyb::k_flow<T, NC, kFwd>, (int)smem));
-    HYB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hyb::k_flow<T, NC, kFwd>, hyb::kThreads,
+    HYB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, hyb::k_flow<T, NC, kFwd>, hyb::kFlowThreads,
                                                            (size_t)smem));
     if (per_sm < 1)
         return HYB_TOO_LARGE;
     const int64_t len = S.dof_off[S.n] * nrhs;
     DevSym ds = h->ds;
-    const T *wbuf = late_blocks<T>(h), *dinv = solve_dinv<T>(h);
+    const T *wbuf = late_blocks<T>(h);
     hyb::Tagged<T> *ytag = scr, *ztag = scr + len, *ptag = scr + 2 * len;
-    int64_t items = (int64_t)(kFwd ? S.fwd_item_p.size() : S.bwd_item_p.size()), withhold = kFwd ? h->withhold_slot : -1;
+    int64_t groups = (int64_t)(kFwd ? S.fwd_item_p.size() : S.bwd_item_p.size()), withhold = kFwd ? h->withhold_slot : -1;
     int mp = max_pivot(S), *status = h->d_solve_status;
     uint64_t wait_ns = h->wait_ns;
-    void *args[] = {&ds,  (void *)&slab, &wbuf, &y,  &ytag,  &ztag,     &ptag,   &dinv,
-                    &tag, &items,        &nrhs, &mp, &stage, &withhold, &status, &wait_ns};
-    const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(items, (int64_t)per_sm * sm_count()));
-    HYB_CUDA(cudaLaunchCooperativeKernel((const void *)hyb::k_flow<T, NC, kFwd>, dim3(grid), dim3(hyb::kThreads), args,
+    // CTAs for the late items (two blocks each) and for the groups (up to eight), in proportion to their
+    // blocks, but with at least an eighth of the CTAs for either kind
+    const int64_t ctas = (int64_t)per_sm * sm_count();
+    int64_t want = ctas * 2 * S.n / (2 * S.n + 8 * groups);
+    want = std::min(S.n, std::max(std::min(want, ctas - ctas / 8), ctas / 8));
+    int late = (int)(groups == 0 ? std::min(S.n, ctas) : std::max<int64_t>(1, want));
+    const unsigned grid = (unsigned)(late + std::min(groups, ctas - late));
+    void *args[] = {&ds,   (void *)&slab, &wbuf, &y,  &ytag,  &ztag,     &ptag,   &tag,
+                    &late, &groups,       &nrhs, &mp, &stage, &withhold, &status, &wait_ns};
+    HYB_CUDA(cudaLaunchCooperativeKernel((const void *)hyb::k_flow<T, NC, kFwd>, dim3(grid), dim3(hyb::kFlowThreads), args,
                                          (size_t)smem, h->stream));
     return HYB_SUCCESS;
 }

@@ -14,12 +14,13 @@ namespace hyb
 constexpr int64_t kBlockAlign = 32;
 
 // Solve (hyb_solve.cuh): early blocks of a pivot's row per item, late blocks of it, and the rows of the
-// pivots that keep W = D^{-1} L for the late blocks. Smaller pivots substitute in less time than
-// the product with W would save; larger ones do not fit k_late.
+// pivots that keep W = D^{-1} L for the late blocks (and X = D^{-1}). Larger pivots do not fit k_late;
+// FP64 solves use them from kFlowLateMin rows on (flow_uses_w).
 constexpr int kFlowGroup = 8;
 constexpr int kFlowLate = 2;
 constexpr int kFlowLateMin = 16;
 constexpr int kFlowLateMax = 128;
+constexpr int kFlowInvMax = 64; // largest of them with X: eight of its values per thread
 constexpr int kFlowPad = 32; // elements a W block is padded to
 
 // Result of the symbolic phase: the reference's elimination replayed on the block
@@ -61,18 +62,19 @@ struct Symbolic
     std::vector<int64_t> upd2_pref; // [n+1] prefix of ceil(|lower column| / 2) * |upper row| (row pairs)
     std::vector<int64_t> split_pref; // [n+1] prefix of n_lc + n_up: blocks whose BF16 split a tensor-core level stages
     std::vector<int64_t> tc_pref;    // [n+1] prefix of n_lc * ceil(n_up / 2): tensor-core update tiles
-    std::vector<int64_t> fwdu_pref; // [n+1] prefix of forward solve items (early groups + the late item)
+    std::vector<int64_t> fwdu_pref; // [n+1] prefix of the early groups of lower blocks (forward solve items)
     std::vector<int32_t> fwd_item_p; // [fwdu_pref[n]] pivot slot of each forward item
-    std::vector<int32_t> bwd_item_p; // backward items (levels descending)
+    std::vector<int32_t> bwd_item_p; // backward items (early groups of upper blocks, levels descending)
+    std::vector<int32_t> bwd_slot;   // [n] pivot slots, levels descending
     std::vector<int64_t> bwd_first;  // [n] first backward item of each pivot slot
     std::vector<int64_t> bwd_lvl;    // [L+1] first backward item of level l (levels descending), [L]: unused
-    std::vector<int64_t> fwd_rows;  // [n+1] prefix of items * pivot size, padded to 4 (scratch rows)
+    std::vector<int64_t> fwd_rows;  // [n+1] prefix of (groups + 1) * pivot size, padded to 4 (scratch rows; 0: no lower blocks)
     std::vector<int64_t> bwd_rows;  // [n+1] the same, backward
-    std::vector<int64_t> w_off;     // [n] offset of a row's W blocks, one after the other, -1 where it has none
-    std::vector<int32_t> w_row, w_blk; // per W block: block row, filled index of the lower block
-    std::vector<int64_t> w_out;     // per W block: its offset
-    int64_t w_elems = 0;            // scalars of all W blocks (padded)
-    int32_t w_cols = 0;             // widest W block
+    std::vector<int64_t> w_off;     // [n] offset of a row's X = D^{-1}, then its W blocks, -1 where it has none
+    std::vector<int32_t> w_row, w_blk; // per X or W block: block row, filled index of the lower block (-1: X)
+    std::vector<int64_t> w_out;     // per X or W block: its offset
+    int64_t w_elems = 0;            // scalars of all X and W blocks (padded)
+    int32_t w_cols = 0;             // widest of them
     std::vector<int32_t> inv_idx;   // [n] slot of a 64-row block row's FP32 diagonal inverse (-1: other sizes)
     std::vector<int32_t> inv_row;   // [n_inv] block row of each inverse slot
     int64_t n_inv = 0;              // block rows of 64

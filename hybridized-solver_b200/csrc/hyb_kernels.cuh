@@ -42,11 +42,12 @@ struct DevSym
     const int64_t *fwdu_pref;
     const int32_t *fwd_item_p; // forward solve: pivot slot of item j (fwdu_pref order)
     const int32_t *bwd_item_p; // backward solve: pivot slot of item j (levels descending)
+    const int32_t *bwd_slot;   // [n] pivot slots, levels descending
     const int64_t *bwd_first;  // [n] first backward item of pivot slot p
     const int64_t *fwd_rows;
     const int64_t *bwd_rows;
-    const int64_t *w_off; // [n] offset of a row's W blocks (Symbolic::w_off), -1: none
-    const int32_t *w_row; // [W blocks] block row, filled index of the lower block and offset of each
+    const int64_t *w_off; // [n] offset of a row's X and W blocks (Symbolic::w_off), -1: none
+    const int32_t *w_row; // [X and W blocks] block row, filled index of the lower block (-1: X) and offset
     const int32_t *w_blk;
     const int64_t *w_out;
     const int32_t *inv_idx; // [n] slot of a 64-row block row's FP32 diagonal inverse (-1: none)
@@ -1577,219 +1578,9 @@ __device__ __forceinline__ bool last_ticket(int *tickets, int64_t p, int64_t npa
     return true;
 }
 
-// Substitution with a factored diagonal block D (unit L below, U on and above the
-// diagonal; row stride ldd) for column r of acc (m x nrhs, shared memory), by one warp:
-// x <- U^{-1} L^{-1} x, as matrix_lu_solve (src/blocks.c:285-316) in right-looking order.
-// The vector stays in registers -- lane l holds rows l + 32 t, t < R. Pivots are taken
-// four per round: their four current values are shuffled at once, every lane finishes the
-// 4x4 triangle with broadcast coefficients, then applies the four updates to the rows it
-// holds, so a round costs one shuffle latency for four pivots. Each row sees the same
-// fused multiply-adds in the same order as with one pivot per round, and registers wholly
-// before (after) the round's 32-row group take no (unmasked) updates.
-template <int R, typename T, typename V>
-__device__ __forceinline__ void warp_lu_solve(const T *d, int ldd, int m, V *acc, int r, int nrhs)
-{
-    const int lane = threadIdx.x & 31;
-    V x[R], rcp[R];
-    int rr[R];
-#pragma unroll
-    for (int t = 0; t < R; ++t)
-    {
-        const int row = lane + 32 * t;
-        rr[t] = min(row, m - 1);
-        x[t] = row < m ? acc[rr[t] * nrhs + r] : V(0);
-        rcp[t] = V(1) / (V)d[(int64_t)rr[t] * ldd + rr[t]];
-    }
-    // ---- forward, unit lower
-#pragma unroll
-    for (int tb = 0; tb < R; ++tb)
-    {
-        const int n_i = min(32, m - 32 * tb);
-        int il = 0;
-        for (; il + 4 <= n_i; il += 4)
-        {
-            const int i = 32 * tb + il;
-            V c[R][4];
-#pragma unroll
-            for (int t = 0; t < R; ++t)
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    c[t][q] = t >= tb ? (V)d[(int64_t)rr[t] * ldd + i + q] : V(0);
-            const V l10 = (V)d[(int64_t)(i + 1) * ldd + i], l20 = (V)d[(int64_t)(i + 2) * ldd + i];
-            const V l21 = (V)d[(int64_t)(i + 2) * ldd + i + 1], l30 = (V)d[(int64_t)(i + 3) * ldd + i];
-            const V l31 = (V)d[(int64_t)(i + 3) * ldd + i + 1], l32 = (V)d[(int64_t)(i + 3) * ldd + i + 2];
-            V a0 = __shfl_sync(0xffffffffu, x[tb], il), a1 = __shfl_sync(0xffffffffu, x[tb], il + 1);
-            V a2 = __shfl_sync(0xffffffffu, x[tb], il + 2), a3 = __shfl_sync(0xffffffffu, x[tb], il + 3);
-            a1 -= l10 * a0;
-            a2 -= l20 * a0;
-            a2 -= l21 * a1;
-            a3 -= l30 * a0;
-            a3 -= l31 * a1;
-            a3 -= l32 * a2;
-            const V av[4] = {a0, a1, a2, a3};
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-#pragma unroll
-                for (int t = 0; t < R; ++t)
-                {
-                    if (t < tb)
-                        continue;
-                    if (t == tb)
-                        x[t] -= (lane > il + q ? c[t][q] : V(0)) * av[q];
-                    else
-                        x[t] -= (lane + 32 * t < m ? c[t][q] : V(0)) * av[q];
-                }
-        }
-        for (; il < n_i; ++il)
-        {
-            const int i = 32 * tb + il;
-            const V xi = __shfl_sync(0xffffffffu, x[tb], il);
-#pragma unroll
-            for (int t = 0; t < R; ++t)
-            {
-                const int row = lane + 32 * t;
-                const V c = (V)d[(int64_t)rr[t] * ldd + i];
-                x[t] -= (row > i && row < m ? c : V(0)) * xi;
-            }
-        }
-    }
-    // ---- backward, upper with the diagonal
-#pragma unroll
-    for (int tb = R - 1; tb >= 0; --tb)
-    {
-        const int n_i = min(32, m - 32 * tb);
-        int il = n_i - 1;
-        for (; il >= 3; il -= 4)
-        {
-            const int i = 32 * tb + il;
-            V c[R][4];
-#pragma unroll
-            for (int t = 0; t < R; ++t)
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    c[t][q] = t <= tb ? (V)d[(int64_t)rr[t] * ldd + i - q] : V(0);
-            const V u10 = (V)d[(int64_t)(i - 1) * ldd + i], u20 = (V)d[(int64_t)(i - 2) * ldd + i];
-            const V u21 = (V)d[(int64_t)(i - 2) * ldd + i - 1], u30 = (V)d[(int64_t)(i - 3) * ldd + i];
-            const V u31 = (V)d[(int64_t)(i - 3) * ldd + i - 1], u32 = (V)d[(int64_t)(i - 3) * ldd + i - 2];
-            const V r0 = __shfl_sync(0xffffffffu, rcp[tb], il), r1 = __shfl_sync(0xffffffffu, rcp[tb], il - 1);
-            const V r2 = __shfl_sync(0xffffffffu, rcp[tb], il - 2), r3 = __shfl_sync(0xffffffffu, rcp[tb], il - 3);
-            V a0 = __shfl_sync(0xffffffffu, x[tb], il), a1 = __shfl_sync(0xffffffffu, x[tb], il - 1);
-            V a2 = __shfl_sync(0xffffffffu, x[tb], il - 2), a3 = __shfl_sync(0xffffffffu, x[tb], il - 3);
-            const V f0 = a0 * r0;
-            a1 -= u10 * f0;
-            const V f1 = a1 * r1;
-            a2 -= u20 * f0;
-            a2 -= u21 * f1;
-            const V f2 = a2 * r2;
-            a3 -= u30 * f0;
-            a3 -= u31 * f1;
-            a3 -= u32 * f2;
-            const V f3 = a3 * r3;
-            const V fv[4] = {f0, f1, f2, f3};
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-#pragma unroll
-                for (int t = 0; t < R; ++t)
-                {
-                    if (t > tb)
-                        continue;
-                    if (t == tb)
-                        x[t] -= (lane < il - q ? c[t][q] : V(0)) * fv[q];
-                    else
-                        x[t] -= c[t][q] * fv[q];
-                }
-            x[tb] = lane == il ? f0 : x[tb];
-            x[tb] = lane == il - 1 ? f1 : x[tb];
-            x[tb] = lane == il - 2 ? f2 : x[tb];
-            x[tb] = lane == il - 3 ? f3 : x[tb];
-        }
-        for (; il >= 0; --il)
-        {
-            const int i = 32 * tb + il;
-            const V xi = __shfl_sync(0xffffffffu, x[tb] * rcp[tb], il);
-            if (lane == il)
-                x[tb] = xi;
-#pragma unroll
-            for (int t = 0; t < R; ++t)
-            {
-                const int row = lane + 32 * t;
-                const V c = (V)d[(int64_t)rr[t] * ldd + i];
-                x[t] -= (row < i ? c : V(0)) * xi;
-            }
-        }
-    }
-#pragma unroll
-    for (int t = 0; t < R; ++t)
-    {
-        const int row = lane + 32 * t;
-        if (row < m)
-            acc[row * nrhs + r] = x[t];
-    }
-}
-
-// One pivot per round (blocks of 65 to 128 rows, where four-pivot rounds would need more
-// registers than the kernels have): step i broadcasts x_i, each step's coefficients are
-// loaded one step ahead.
-template <int R, typename T, typename V>
-__device__ __forceinline__ void warp_lu_solve1(const T *d, int ldd, int m, V *acc, int r, int nrhs)
-{
-    const int lane = threadIdx.x & 31;
-    V x[R], rcp[R];
-#pragma unroll
-    for (int t = 0; t < R; ++t)
-    {
-        const int row = lane + 32 * t, rr = min(row, m - 1);
-        x[t] = row < m ? acc[rr * nrhs + r] : V(0);
-        rcp[t] = V(1) / (V)d[(int64_t)rr * ldd + rr];
-    }
-#pragma unroll
-    for (int tb = 0; tb < R; ++tb)
-    {
-        const int n_i = min(32, m - 32 * tb);
-#pragma unroll 2
-        for (int il = 0; il < n_i; ++il)
-        {
-            const int i = 32 * tb + il;
-            const V xi = __shfl_sync(0xffffffffu, x[tb], il);
-#pragma unroll
-            for (int t = 0; t < R; ++t)
-            {
-                const int row = lane + 32 * t, rr = min(row, m - 1);
-                const V c = (V)d[(int64_t)rr * ldd + i];
-                x[t] -= (row > i && row < m ? c : V(0)) * xi;
-            }
-        }
-    }
-#pragma unroll
-    for (int tb = R - 1; tb >= 0; --tb)
-    {
-        const int n_i = min(32, m - 32 * tb);
-#pragma unroll 2
-        for (int il = n_i - 1; il >= 0; --il)
-        {
-            const int i = 32 * tb + il;
-            const V xi = __shfl_sync(0xffffffffu, x[tb] * rcp[tb], il);
-            if (lane == il)
-                x[tb] = xi;
-#pragma unroll
-            for (int t = 0; t < R; ++t)
-            {
-                const int row = lane + 32 * t, rr = min(row, m - 1);
-                const V c = (V)d[(int64_t)rr * ldd + i];
-                x[t] -= (row < i ? c : V(0)) * xi;
-            }
-        }
-    }
-#pragma unroll
-    for (int t = 0; t < R; ++t)
-    {
-        const int row = lane + 32 * t;
-        if (row < m)
-            acc[row * nrhs + r] = x[t];
-    }
-}
-
-// The same for blocks of more than 128 rows, through shared memory.
+// Substitution with a factored diagonal block D (unit L below, U on and above the diagonal; row stride
+// ldd) for column r of acc (m x nrhs, shared memory), by one warp through shared memory: for
+// blocks too large for registers (hyb_solve.cuh has the others).
 template <typename T, typename V>
 __device__ void warp_lu_solve_smem(const T *d, int ldd, int m, V *acc, int r, int nrhs)
 {
@@ -1899,49 +1690,6 @@ template <typename V> __device__ void sum_partials(const V *part, int64_t nparts
         const V v = sum_strided(part, nparts, E, 1, 0, e2);
         out[e2] = v;
     }
-}
-
-// Explicit inverses of the 64x64 diagonal blocks for the FP32 solves inside the mixed
-// form's refinement, where the inner solve only has to be a good approximation (the FP64
-// residual decides convergence): X = D^{-1} from D's LU factors, column j of X by thread
-// j as U^{-1} (L^{-1} e_j) with the substitution's arithmetic (unit L, multiply by the
-// reciprocal of U's diagonal), stored transposed (xt[j * 64 + i] = X(i, j)) so the
-// forward solve's register layout reads it directly. One CTA per inverse slot.
-constexpr int kInvThreads = 64;
-template <typename T>
-__global__ void __launch_bounds__(kInvThreads) k_diag_inv64(DevSym S, const T *__restrict__ slab, T *__restrict__ dinv)
-{
-    __shared__ __align__(16) T sd[64 * 64];
-    const int32_t slot = blockIdx.x;
-    const int64_t k = S.inv_row[slot];
-    const T *gd = slab + S.blk_off[S.diag_pos[k]];
-    for (int i = threadIdx.x; i < 64 * 64; i += blockDim.x)
-        sd[i] = gd[i];
-    __syncthreads();
-    const int j = threadIdx.x;
-    T y[64];
-#pragma unroll
-    for (int i = 0; i < 64; ++i)
-    {
-        T s = i == j ? T(1) : T(0);
-#pragma unroll
-        for (int c = 0; c < i; ++c)
-            s -= sd[i * 64 + c] * y[c];
-        y[i] = s;
-    }
-#pragma unroll
-    for (int i = 63; i >= 0; --i)
-    {
-        T s = y[i];
-#pragma unroll
-        for (int c = i + 1; c < 64; ++c)
-            s -= sd[i * 64 + c] * y[c];
-        y[i] = s * (T(1) / sd[i * 64 + i]);
-    }
-    T *xt = dinv + (int64_t)slot * 4096 + j * 64;
-#pragma unroll
-    for (int i = 0; i < 64; ++i)
-        xt[i] = y[i];
 }
 
 // Threads per row of a product with an m-row block: the largest power of two, at most 32, that leaves a CTA's

@@ -7,21 +7,26 @@
 // y_{k-1} and the departure of y_k. Both are kept short:
 //  - a vector travels as tagged values -- value and tag of this solve and direction in one
 //    store -- so a reader that sees the tag has the value: no fence, no flag, no second read;
-//  - the nearest sources' blocks ("late": up to two) are handled apart from the others. Pivots of 16
+//  - the nearest sources' blocks ("late": up to two) are handled apart from the others. Pivots of up
 //    to 128 rows keep W(k,s) = D_k^{-1} L(k,s) for them (k_late, after the factorization), so that
 //    y_k = D_k^{-1} (y_k - sum of the others) - sum_late W(k,s) y_s: the substitution with D_k is
 //    done while the late sources are still on their way, and only one product is left when
 //    the last one arrives. W is solved for like U, with the same bound on the result's error as
-//    substituting afterwards;
+//    substituting afterwards; D_k^{-1} itself is applied as a product with the inverse and, in
+//    FP64, one correction (flow_diag_solve);
 //  - the other ("early") blocks go in groups of up to eight to a CTA each, which adds their products in
 //    registers as the sources arrive; the group nearest the pivot collects the others' sums.
-// Measured on a B200, both directions, one right-hand side: see k_flow.
+// Measured on a B200, both directions, one right-hand side, before (flags, D_k substituted on the chain) and
+// after: 40x40 p=8 FP64 21.9 to 8.5 ms, 64x64 56 to 23.5 ms, 16x16 p=4 2.3 to 1.1 ms; two FP32
+// solves of a mixed step at 31x31 16.2 to 8.3 ms, at 96x96 169 to 105 ms. Of a hop's 1.8 us about
+// 0.4 us is the trip through L2, 0.95 us the additions, their reduction and the stores.
 //
 // Two forms with the same arithmetic (bit-identical results): k_flow, one cooperative launch per
 // direction, and k_stage, one launch per level and direction.
 #pragma once
 
 #include "hyb_front.cuh"
+#include "hyb_internal.h"
 
 namespace hyb
 {
@@ -76,19 +81,21 @@ __device__ __forceinline__ bool tag_load(const Tagged<float> *p, int tag, float 
 template <typename T>
 __device__ __forceinline__ bool tag_wait(const Tagged<T> *p, int tag, T &v, bool pause, int *status, uint64_t wait_ns)
 {
-    if (tag_load(p, tag, v))
-        return true;
-    const uint64_t t0 = global_ns();
+    uint64_t t0 = 0;
     for (;;)
     {
-        for (int i = 0; i < 32; ++i)
+        // reading the timer is slower than a trip to L2: not before 10 us or so have passed
+        for (int i = 0; i < 64; ++i)
         {
-            if (pause)
-                __nanosleep(40);
             if (tag_load(p, tag, v))
                 return true;
+            if (pause)
+                __nanosleep(40);
         }
-        if (schedule_aborted(status) || global_ns() - t0 > wait_ns)
+        const uint64_t t = global_ns();
+        if (t0 == 0)
+            t0 = t;
+        if (schedule_aborted(status) || t - t0 > wait_ns)
         {
             atomicOr(status + ST_TIMEOUT, 1);
             return false;
@@ -107,23 +114,52 @@ struct FlowRow
     int m, nb, ne, ng;
 };
 
-template <bool kFwd> __device__ __forceinline__ FlowRow flow_row(const DevSym &S, int64_t k)
+// Whether the solves of precision T use X and W of an m-row pivot (Symbolic::w_off). FP64 leaves pivots of
+// fewer than 16 rows to substitution, which takes them little time and whose roundings are then
+// those of the dense block kernels.
+template <typename T> __host__ __device__ constexpr bool flow_uses_w(int m)
+{
+    return std::is_same_v<T, float> || m >= kFlowLateMin;
+}
+
+template <bool kFwd, typename T> __device__ __forceinline__ FlowRow flow_row(const DevSym &S, int64_t k)
 {
     FlowRow f;
     const int64_t d = S.diag_pos[k];
     f.k = k;
     f.m = S.size[k];
-    f.w = kFwd ? S.w_off[k] : -1;
+    f.w = kFwd && flow_uses_w<T>(f.m) ? S.w_off[k] : -1;
     f.base = kFwd ? S.row_ptr[k] : d + 1;
     f.nb = (int)(kFwd ? d - f.base : S.row_ptr[k + 1] - f.base);
-    f.ne = f.nb - min(f.nb, kFwd && f.w < 0 ? 1 : kFlowLate);
+    f.ne = f.nb - min(f.nb, kFlowLate);
     f.ng = (f.ne + kFlowGroup - 1) / kFlowGroup;
     return f;
 }
 
-// Up to 16 columns of every row of one block in registers: thread t holds, of row r0 + t / tpr, the
+// Loads that stay where they are written: the compiler moves ordinary ones behind the wait for the source
+// that they are there to overlap (a hop then took 3 us more).
+__device__ __forceinline__ double load_now(const double *p)
+{
+    double v;
+    asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+
+__device__ __forceinline__ float load_now(const float *p)
+{
+    float v;
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+
+// One CTA of 512 threads per SM: a piece of 4,096 values takes eight registers of each, so the two pieces
+// that an item holds leave room for all else (with 256 threads and twice the values, two CTAs
+// to an SM, a hop waited for 500 bytes of spilled registers to come back from L2).
+constexpr int kFlowThreads = 512;
+
+// Up to eight columns of every row of one block in registers: thread t holds, of row r0 + t / tpr, the
 // columns c0 + t % tpr + tpr c.
-constexpr int kFlowRegs = 16;
+constexpr int kFlowRegs = 8;
 template <typename T> struct FlowBlock
 {
     T v[kFlowRegs];
@@ -144,24 +180,19 @@ __device__ __forceinline__ void flow_load(FlowBlock<T> &g, const DevSym &S, cons
     const T *p = slab + S.blk_off[blk];
     if (kFwd && f.w >= 0 && i >= f.ne)
     {
-        p = wbuf + f.w;
+        p = wbuf + f.w + (f.m <= kFlowInvMax ? (f.m * f.m + kFlowPad - 1) / kFlowPad * kFlowPad : 0);
         for (int e = f.ne; e < i; ++e) // the late blocks before it
             p += (f.m * S.size[S.cols[f.base + e]] + kFlowPad - 1) / kFlowPad * kFlowPad;
     }
     const int row = r0 + (int)threadIdx.x / tpr, q = c0 + ((int)threadIdx.x & (tpr - 1));
     p += (int64_t)row * g.K + q;
-    const bool in = row < f.m;
-    if (c0 + kFlowRegs * tpr <= g.K)
-    {
+    const int left = row < f.m ? g.K - q : 0; // columns of this thread's row from its first on
 #pragma unroll
-        for (int c = 0; c < kFlowRegs; ++c)
-            g.v[c] = in ? p[c * tpr] : T(0);
-    }
-    else
+    for (int c = 0; c < kFlowRegs; ++c)
     {
-#pragma unroll
-        for (int c = 0; c < kFlowRegs; ++c)
-            g.v[c] = in && q + c * tpr < g.K ? p[c * tpr] : T(0);
+        g.v[c] = T(0);
+        if (c * tpr < left)
+            g.v[c] = load_now(p + c * tpr);
     }
 }
 
@@ -201,11 +232,19 @@ template <typename T, int NC> __device__ __forceinline__ void flow_reduce(FlowSu
     }
 }
 
+// D as it is staged for flow_lu: rows and columns rounded up to eight and continued by the identity, row
+// stride odd (the rows a warp touches sit in different banks).
+__host__ __device__ constexpr int flow_rows(int m)
+{
+    return (m + 7) / 8 * 8;
+}
+
 // Shared memory of a CTA of k_flow and k_stage, in values of T: two source vectors, a vector of the pivot's
-// that is worked on, one that is kept, partial products of an inverse, and the diagonal block.
+// that is worked on, one that is kept, and the diagonal block.
 template <typename T> struct FlowSmem
 {
-    T *y[2], *acc, *z, *part, *d;
+    T *y, *acc, *z, *d; // y: two vectors of len values
+    int len;
 };
 
 template <typename T> __device__ __forceinline__ FlowSmem<T> flow_smem(int max_m, int nc)
@@ -213,123 +252,267 @@ template <typename T> __device__ __forceinline__ FlowSmem<T> flow_smem(int max_m
     extern __shared__ __align__(16) unsigned char smem_raw[];
     FlowSmem<T> s;
     T *p = reinterpret_cast<T *>(smem_raw);
-    s.y[0] = p;
-    s.y[1] = s.y[0] + max_m * nc;
-    s.acc = s.y[1] + max_m * nc;
-    s.z = s.acc + max_m * nc;
-    s.part = s.z + max_m * nc;
-    s.d = s.part + kThreads;
+    s.len = flow_rows(max_m) * nc;
+    s.y = p;
+    s.acc = s.y + 2 * s.len;
+    s.z = s.acc + s.len;
+    s.d = s.z + s.len;
     return s;
 }
 
 template <typename T> __host__ __device__ constexpr int64_t flow_smem_bytes(int max_m, int nc, bool stage)
 {
-    return ((int64_t)4 * max_m * nc + kThreads + (stage ? (int64_t)max_m * (max_m | 1) : 0)) * (int64_t)sizeof(T);
+    const int mp = flow_rows(max_m);
+    return ((int64_t)4 * mp * nc + (stage ? (int64_t)mp * (mp | 1) : 0)) * (int64_t)sizeof(T);
 }
 
-// What a CTA prepares to apply D_k^{-1}: k's inverse in registers where the factorization left one (dinv
-// set, 64 rows), else D_k in shared memory (stage) with an odd row stride.
+// What a CTA prepares to apply D_k^{-1}: of a pivot with an inverse X (up to 64 rows; k_late) its share of
+// X in registers, and (FP64, or without an inverse) D_k in shared memory (stage) with an odd row stride.
 template <typename T> struct FlowDiag
 {
-    static constexpr int kInv = std::is_same_v<T, float> ? kFlowRegs : 1; // only FP32 factors have inverses
-    T inv[kInv];
-    bool has_inv;
+    T x[kFlowRegs];
 };
 
 template <typename T>
 __device__ __forceinline__ void flow_diag_load(FlowDiag<T> &g, const DevSym &S, const T *__restrict__ slab,
-                                               const T *__restrict__ dinv, int64_t k, int m, T *sd, int stage)
+                                               const T *__restrict__ wbuf, int64_t k, int m, int tpr, T *sd, int stage)
 {
-    g.has_inv = std::is_same_v<T, float> && dinv && S.inv_idx[k] >= 0;
-    if (g.has_inv)
+    const int64_t w = flow_uses_w<T>(m) ? S.w_off[k] : -1;
+    const int row = (int)threadIdx.x / tpr, q = (int)threadIdx.x & (tpr - 1);
+    const bool inv = w >= 0 && m <= kFlowInvMax;
+    if (inv)
     {
-        const T *x = dinv + (int64_t)S.inv_idx[k] * 4096;
 #pragma unroll
-        for (int q = 0; q < FlowDiag<T>::kInv; ++q)
-            g.inv[q] = x[q * kThreads + threadIdx.x];
+        for (int c = 0; c < kFlowRegs; ++c)
+            g.x[c] = row < m && q + c * tpr < m ? wbuf[w + row * m + q + c * tpr] : T(0);
     }
-    else if (stage)
+    if (stage && m <= kFlowLateMax && (!inv || std::is_same_v<T, double>))
     {
         const T *gd = slab + S.blk_off[S.diag_pos[k]];
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = kThreads / 32;
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = kFlowThreads / 32;
+        const int mp = flow_rows(m), ld = mp | 1;
 #pragma unroll 4
-        for (int r = warp; r < m; r += nw)
-            for (int c = lane; c < m; c += 32)
-                sd[r * (m | 1) + c] = gd[r * m + c];
+        for (int r = warp; r < mp; r += nw)
+            for (int c = lane; c < mp; c += 32)
+                sd[r * ld + c] = r < m && c < m ? gd[r * m + c] : T(r == c);
+    }
+}
+
+// Products with m x m blocks, m <= 64, by every thread of the CTA, a barrier after them; in, out: m rows, nc of
+// NC columns in shared memory. kind 0: out = X in; 1: out += X in; 2: out = U in; 3: out = b - L in with
+// L unit lower, D = L U in d (row stride ld).
+template <typename T, int NC, int kKind>
+__device__ __forceinline__ void flow_product(const FlowDiag<T> &g, const T *d, int ld, int m, int tpr, const T *in,
+                                             const T *b, T *out, int nc)
+{
+    const int row = (int)threadIdx.x / tpr, q = (int)threadIdx.x & (tpr - 1);
+    T e[kFlowRegs];
+    if (kKind < 2)
+    {
+#pragma unroll
+        for (int c = 0; c < kFlowRegs; ++c)
+            e[c] = g.x[c];
+    }
+    else
+    {
+#pragma unroll
+        for (int c = 0; c < kFlowRegs; ++c)
+        {
+            const int col = q + c * tpr;
+            e[c] = row < m && col < m && (kKind == 2 ? col >= row : col < row) ? d[row * ld + col] : T(0);
+        }
+    }
+    for (int r = 0; r < nc; ++r)
+    {
+        T s[2] = {};
+#pragma unroll
+        for (int c = 0; c < kFlowRegs; ++c)
+            if (q + c * tpr < m)
+                s[c & 1] += e[c] * in[(q + c * tpr) * NC + r];
+        T t = s[0] + s[1];
+        for (int o = tpr >> 1; o > 0; o >>= 1)
+            t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (q == 0 && row < m)
+            out[row * NC + r] = kKind == 3   ? b[row * NC + r] - (in[row * NC + r] + t)
+                                : kKind == 1 ? out[row * NC + r] + t
+                                             : t;
+    }
+    __syncthreads();
+}
+
+// x <- U^{-1} L^{-1} x, as matrix_lu_solve (src/blocks.c:285-316) in right-looking order, for one column x
+// (stride xs, zero in the rows beyond the block) by one warp: lane l holds rows l + 32 t, t < R.
+// Eight pivots per round: their values go to every lane, which finishes the 8x8 triangle for
+// itself, then applies the eight updates to its rows. Each row sees the fused multiply-adds
+// of one pivot after the other; a round costs one shuffle latency for eight pivots.
+template <int R, typename T> __device__ __forceinline__ void flow_lu(const T *d, int mp, T *x, int xs)
+{
+    const int lane = threadIdx.x & 31, ld = mp | 1;
+    T v[R], rcp[R];
+#pragma unroll
+    for (int t = 0; t < R; ++t)
+    {
+        const int row = lane + 32 * t;
+        v[t] = row < mp ? x[row * xs] : T(0);
+        rcp[t] = row < mp ? T(1) / d[row * (ld + 1)] : T(0);
+    }
+#pragma unroll
+    for (int tb = 0; tb < R; ++tb)
+#pragma unroll 1
+        for (int il = 0; il < 32 && 32 * tb + il < mp; il += 8)
+        {
+            const T *di = d + (32 * tb + il) * (ld + 1); // the 8x8 block
+            T a[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                a[j] = __shfl_sync(0xffffffffu, v[tb], il + j);
+#pragma unroll
+            for (int j = 0; j < 7; ++j)
+#pragma unroll
+                for (int i = j + 1; i < 8; ++i)
+                    a[i] -= di[i * ld + j] * a[j];
+#pragma unroll
+            for (int t = tb; t < R; ++t)
+            {
+                const int row = lane + 32 * t;
+                const T *c = d + min(row, mp - 1) * ld + 32 * tb + il;
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (t > tb || lane > il + j)
+                        v[t] -= c[j] * a[j];
+            }
+        }
+#pragma unroll
+    for (int tb = R - 1; tb >= 0; --tb)
+#pragma unroll 1
+        for (int il = min(24, mp - 32 * tb - 8); il >= 0; il -= 8)
+        {
+            const T *di = d + (32 * tb + il) * (ld + 1);
+            T a[8], r[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+            {
+                a[j] = __shfl_sync(0xffffffffu, v[tb], il + j);
+                r[j] = __shfl_sync(0xffffffffu, rcp[tb], il + j);
+            }
+#pragma unroll
+            for (int j = 7; j >= 0; --j)
+            {
+                a[j] *= r[j];
+#pragma unroll
+                for (int i = 0; i < j; ++i)
+                    a[i] -= di[i * ld + j] * a[j];
+                if (lane == il + j)
+                    v[tb] = a[j];
+            }
+#pragma unroll
+            for (int t = 0; t <= tb; ++t)
+            {
+                const T *c = d + (lane + 32 * t) * ld + 32 * tb + il;
+#pragma unroll
+                for (int j = 7; j >= 0; --j)
+                    if (t < tb || lane < il)
+                        v[t] -= c[j] * a[j];
+            }
+        }
+#pragma unroll
+    for (int t = 0; t < R; ++t)
+    {
+        const int row = lane + 32 * t;
+        if (row < mp)
+            x[row * xs] = v[t];
     }
 }
 
 // acc <- D^{-1} acc for nc of NC columns by substitution (a function of its own: its registers are not
-// needed while blocks are held).
+// needed while blocks are held). d: staged, or (null) the block in global memory.
 template <typename T, int NC>
-__device__ __noinline__ void flow_substitute(const T *d, int ldd, int m, T *acc, int nc)
+__device__ __noinline__ void flow_substitute(const T *d, const T *gd, int m, T *acc, int nc)
 {
-    for (int r = threadIdx.x >> 5; r < nc; r += kThreads / 32)
+    const int mp = flow_rows(m);
+    for (int r = threadIdx.x >> 5; r < nc; r += kFlowThreads / 32)
     {
-        if (m <= 32)
-            warp_lu_solve<1>(d, ldd, m, acc, r, NC);
+        if (!d)
+            warp_lu_solve_smem(gd, m, m, acc, r, NC);
+        else if (m <= 32)
+            flow_lu<1>(d, mp, acc + r, NC);
         else if (m <= 64)
-            warp_lu_solve<2>(d, ldd, m, acc, r, NC);
-        else if (m <= 96)
-            warp_lu_solve1<3>(d, ldd, m, acc, r, NC);
-        else if (m <= 128)
-            warp_lu_solve1<4>(d, ldd, m, acc, r, NC);
+            flow_lu<2>(d, mp, acc + r, NC);
         else
-            warp_lu_solve_smem(d, ldd, m, acc, r, NC);
+            flow_lu<4>(d, mp, acc + r, NC);
     }
 }
 
 // acc <- D_k^{-1} acc for nc of NC columns, by every thread of the CTA; acc is complete and in place after
-// a barrier on both sides.
+// a barrier on both sides. With an inverse: v = X acc, in FP64 corrected once by the residual of its
+// own system, v += X (acc - L (U v)), which makes the solution as accurate as one by substitution
+// (fixed-precision refinement: backward stable while cond(D) eps < 1) with four products in
+// the place of 2 m dependent steps: 16,000 cycles for 64 rows by substitution. FP32 solves only
+// have to approximate and take v as it is. Without: substitution. tmp: two vectors.
 template <typename T, int NC>
 __device__ __forceinline__ void flow_diag_solve(const FlowDiag<T> &g, const DevSym &S, const T *__restrict__ slab,
-                                                int64_t k, int m, T *acc, T *part, const T *sd, int stage, int nc)
+                                                const T *__restrict__ wbuf, int64_t k, int m, int tpr, T *acc, T *tmp,
+                                                int len, const T *sd, int stage, int nc)
 {
     const int tid = threadIdx.x;
-    if constexpr (std::is_same_v<T, float>)
-        if (g.has_inv)
+    const int64_t w = flow_uses_w<T>(m) ? S.w_off[k] : -1;
+    const T *gd = slab + S.blk_off[S.diag_pos[k]];
+    const bool staged = stage && m <= kFlowLateMax;
+    if (w >= 0 && m <= kFlowInvMax)
+    {
+        T *v = tmp, *t = tmp + len;
+        flow_product<T, NC, 0>(g, nullptr, 0, m, tpr, acc, nullptr, v, nc);
+        if constexpr (std::is_same_v<T, double>)
         {
-            // thread t holds X(t mod 64, 4 q + t / 64): four sums per row, added in a fixed order
-            for (int c = 0; c < nc; ++c)
-            {
-                T s = T(0);
-#pragma unroll
-                for (int q = 0; q < kFlowRegs; ++q)
-                    s += g.inv[q] * acc[(4 * q + (tid >> 6)) * NC + c];
-                part[tid] = s;
-                __syncthreads();
-                if (tid < 64)
-                    acc[tid * NC + c] = (part[tid] + part[64 + tid]) + (part[128 + tid] + part[192 + tid]);
-                __syncthreads();
-            }
-            return;
+            const T *d = staged ? sd : gd;
+            const int ld = staged ? (flow_rows(m) | 1) : m;
+            flow_product<T, NC, 2>(g, d, ld, m, tpr, v, nullptr, t, nc);
+            flow_product<T, NC, 3>(g, d, ld, m, tpr, t, acc, acc, nc);
+            flow_product<T, NC, 1>(g, nullptr, 0, m, tpr, acc, nullptr, v, nc);
         }
-    flow_substitute<T, NC>(stage ? sd : slab + S.blk_off[S.diag_pos[k]], stage ? (m | 1) : m, m, acc, nc);
+        for (int e = tid; e < m * NC; e += kFlowThreads)
+            acc[e] = v[e];
+        __syncthreads();
+        return;
+    }
+    const int mp = flow_rows(m);
+    if (staged && mp > m) // the columns' padding
+    {
+        for (int e = m * NC + tid; e < mp * NC; e += kFlowThreads)
+            acc[e] = T(0);
+        __syncthreads();
+    }
+    flow_substitute<T, NC>(staged ? sd : nullptr, gd, m, acc, nc);
     __syncthreads();
 }
 
-// Dataflow substitution, one direction: a cooperative launch in which CTA b takes the items b, b + G, ...
-// in order. Items are ordered by level (forward ascending, backward descending), a pivot's late item
-// last; an item waits only for items before it and all CTAs are resident, so every wait ends; each
-// is also bounded in time. ytag, ztag: dof x nrhs tagged values (the solution so far; a
+// Dataflow substitution, one direction: a cooperative launch in which the first n_late CTAs take the
+// pivots' late items in turn and the others the groups, both in order of the levels (forward
+// ascending, backward descending). An item waits only for items of earlier levels and of its
+// own pivot's groups before it, and all CTAs are resident, so every wait ends; each is also
+// bounded in time. The two kinds have CTAs of their own because a hop takes little more than
+// its instructions do, and those of a path that a CTA takes now and then come from far: with
+// both kinds on every CTA the eight additions after an arrival took 1,400 cycles. ytag, ztag: dof x nrhs tagged values (the solution so far; a
 // pivot's vector without its late sources, forward with D_k^{-1} applied where W exists); ptag:
 // the sums of a pivot's early groups. The blocks of an item stream through two register
 // buffers, the next one loaded while the present one waits for its source.
 // withhold: pivot slot whose ztag is never written (fault injection), or -1.
 template <typename T, int NC, bool kFwd>
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(kFlowThreads, 1)
     k_flow(DevSym S, const T *__restrict__ slab, const T *__restrict__ wbuf, T *__restrict__ y, Tagged<T> *ytag,
-           Tagged<T> *ztag, Tagged<T> *ptag, const T *__restrict__ dinv, int tag, int64_t n_items, int nrhs, int max_m,
+           Tagged<T> *ztag, Tagged<T> *ptag, int tag, int n_late, int64_t n_groups, int nrhs, int max_m,
            int stage, int64_t withhold, int *status, uint64_t wait_ns)
 {
     const FlowSmem<T> sm = flow_smem<T>(max_m, NC);
     const int tid = threadIdx.x;
-    for (int64_t j = blockIdx.x; j < n_items; j += gridDim.x)
+    const bool late = (int)blockIdx.x < n_late;
+    const int64_t n_items = late ? S.n : n_groups, stride = late ? n_late : (int)gridDim.x - n_late;
+    for (int64_t j = late ? (int)blockIdx.x : (int)blockIdx.x - n_late; j < n_items; j += stride)
     {
-        const int64_t p = kFwd ? S.fwd_item_p[j] : S.bwd_item_p[j];
-        const FlowRow f = flow_row<kFwd>(S, S.piv[p]);
-        const int local = (int)(j - (kFwd ? S.fwdu_pref[p] : S.bwd_first[p])), m = f.m;
-        const bool late = local == f.ng, last_group = local == f.ng - 1;
+        const int64_t p = late ? (kFwd ? j : S.bwd_slot[j]) : (kFwd ? S.fwd_item_p[j] : S.bwd_item_p[j]);
+        const FlowRow f = flow_row<kFwd, T>(S, S.piv[p]);
+        const int local = late ? f.ng : (int)(j - (kFwd ? S.fwdu_pref[p] : S.bwd_first[p])), m = f.m;
+        const bool last_group = local == f.ng - 1;
         const int i1 = late ? f.nb : f.ne - (f.ng - 1 - local) * kFlowGroup;
         const int i0 = late ? f.ne : max(0, i1 - kFlowGroup);
         const bool has_w = kFwd && f.w >= 0, held = p == withhold;
@@ -337,29 +520,29 @@ __global__ void __launch_bounds__(kThreads, 2)
         const bool solves = kFwd && (has_w ? last_group || (late && f.ng == 0) : late);
         const int64_t row_off = S.dof_off[f.k] * nrhs;
         Tagged<T> *part = ptag + (kFwd ? S.fwd_rows[p] : S.bwd_rows[p]) * nrhs;
-        const int tpr = gemv_tpr<T>(m), rows = kThreads / tpr, q = tid & (tpr - 1);
+        const int tpr = gemv_tpr<T>(m), rows = kFlowThreads / tpr, q = tid & (tpr - 1);
         FlowDiag<T> dg;
         for (int ch = 0; ch < nrhs; ch += NC)
         {
             const int nc = min(NC, nrhs - ch);
             for (int r0 = 0; r0 < m; r0 += rows)
             {
-                FlowBlock<T> g[2];
+                FlowBlock<T> cur, nxt;
                 if (i0 < i1)
-                    flow_load<kFwd>(g[0], S, f, slab, wbuf, i0, 0, r0, tpr);
+                    flow_load<kFwd>(cur, S, f, slab, wbuf, i0, 0, r0, tpr);
                 if (solves && ch == 0 && r0 == 0)
-                    flow_diag_load(dg, S, slab, dinv, f.k, m, sm.d, stage);
+                    flow_diag_load(dg, S, slab, wbuf, f.k, m, tpr, sm.d, stage);
                 __syncthreads(); // shared memory is free, D_k is staged
                 bool ok = true;
                 if (late && f.ng == 0 && r0 == 0)
                 {
                     // no early blocks: the pivot's own values, solved at once where W exists
-                    for (int e = tid; e < m * nc; e += kThreads)
+                    for (int e = tid; e < m * nc; e += kFlowThreads)
                         sm.acc[e / nc * NC + e % nc] = y[row_off + (int64_t)(e / nc) * nrhs + ch + e % nc];
                     __syncthreads();
                     if (has_w)
-                        flow_diag_solve<T, NC>(dg, S, slab, f.k, m, sm.acc, sm.part, sm.d, stage, nc);
-                    for (int e = tid; e < m * NC; e += kThreads)
+                        flow_diag_solve<T, NC>(dg, S, slab, wbuf, f.k, m, tpr, sm.acc, sm.y, sm.len, sm.d, stage, nc);
+                    for (int e = tid; e < m * NC; e += kFlowThreads)
                         sm.z[e] = sm.acc[e];
                     if (held)
                     {
@@ -369,23 +552,27 @@ __global__ void __launch_bounds__(kThreads, 2)
                 }
                 FlowSum<T, NC> a = {};
                 int par = 0;
-                // one step: prefetch the next piece, wait for this block's source, add
-                auto step = [&](FlowBlock<T> &cur, FlowBlock<T> &nxt) {
+#pragma unroll 1
+                for (bool more = i0 < i1; more;)
+                {
+                    // prefetch the next piece, wait for this block's source, add
                     int ni = cur.i, nc0 = cur.c0 + kFlowRegs * tpr;
                     if (nc0 >= cur.K)
                     {
                         ++ni;
                         nc0 = 0;
                     }
-                    if (ni < i1)
+                    more = ni < i1;
+                    if (more)
                         flow_load<kFwd>(nxt, S, f, slab, wbuf, ni, nc0, r0, tpr);
                     if (cur.c0 == 0)
                     {
                         par ^= 1;
-                        if (cur.i == i1 - 1 && (late ? f.ng > 0 : last_group && f.ng > 1))
+                        const bool last = cur.i == i1 - 1;
+                        if (last && (late ? f.ng > 0 : last_group && f.ng > 1))
                         {
                             // before the item's last source: what the pivot's other items have
-                            for (int e = tid; e < m * nc && ok; e += kThreads)
+                            for (int e = tid; e < m * nc && ok; e += kFlowThreads)
                             {
                                 const int64_t at = (int64_t)(e / nc) * nrhs + ch + e % nc;
                                 T v, s = T(0);
@@ -394,36 +581,37 @@ __global__ void __launch_bounds__(kThreads, 2)
                                 else
                                     for (int h = 0; h < f.ng - 1 && ok; ++h)
                                     {
-                                        ok = tag_wait(part + (int64_t)h * m * nrhs + at, tag, v, true, status, wait_ns);
+                                        ok = tag_wait(part + (int64_t)h * m * nrhs + at, tag, v, false, status, wait_ns);
                                         s = h == 0 ? v : s + v;
                                     }
                                 sm.z[e / nc * NC + e % nc] = s;
                             }
                         }
+                        // The last late source is awaited by every reader of its values; the others, for which
+                        // many CTAs wait at once, by one thread of each until their first value is there.
                         const Tagged<T> *src = ytag + cur.src * nrhs + ch;
-                        for (int e = tid; e < cur.K * nc && ok; e += kThreads)
+                        if (!(late && last))
                         {
                             T v;
-                            ok = tag_wait(src + (int64_t)(e / nc) * nrhs + e % nc, tag, v, !late, status, wait_ns);
-                            sm.y[par][e / nc * NC + e % nc] = v;
+                            if (tid == 0 && ok)
+                                ok = tag_wait(src, tag, v, true, status, wait_ns);
+                            ok = __syncthreads_and(ok) != 0;
+                        }
+                        for (int e = tid; e < cur.K * nc && ok; e += kFlowThreads)
+                        {
+                            T v;
+                            ok = tag_wait(src + (int64_t)(e / nc) * nrhs + e % nc, tag, v, false, status, wait_ns);
+                            sm.y[par * sm.len + e / nc * NC + e % nc] = v;
                         }
                         ok = __syncthreads_and(ok) != 0;
+                        if (!ok)
+                            return; // uniform
                     }
-                    if (ok)
-                        flow_add<T, NC>(a, cur, sm.y[par], tpr);
-                    return ok && ni < i1;
-                };
-                if (i0 < i1)
-                {
-                    while (step(g[0], g[1]) && step(g[1], g[0]))
-                        ;
+                    flow_add<T, NC>(a, cur, sm.y + par * sm.len, tpr);
+                    cur = nxt;
                 }
-                else
-                {
-                    ok = __syncthreads_and(ok) != 0;
-                }
-                if (!ok)
-                    return; // uniform
+                if (i0 >= i1 && __syncthreads_and(ok) == 0)
+                    return;
                 flow_reduce<T, NC>(a, tpr);
                 const int row = r0 + tid / tpr;
                 if (q == 0 && row < m)
@@ -466,8 +654,8 @@ __global__ void __launch_bounds__(kThreads, 2)
             if (solves && !(late && has_w))
             {
                 __syncthreads();
-                flow_diag_solve<T, NC>(dg, S, slab, f.k, m, sm.acc, sm.part, sm.d, stage, nc);
-                for (int e = tid; e < m * nc; e += kThreads)
+                flow_diag_solve<T, NC>(dg, S, slab, wbuf, f.k, m, tpr, sm.acc, sm.y, sm.len, sm.d, stage, nc);
+                for (int e = tid; e < m * nc; e += kFlowThreads)
                 {
                     const int64_t at = (int64_t)(e / nc) * nrhs + ch + e % nc;
                     const T v = sm.acc[e / nc * NC + e % nc];
@@ -480,26 +668,28 @@ __global__ void __launch_bounds__(kThreads, 2)
     }
 }
 
-// The same, one level and direction per launch: CTA b takes item first + b of the level's items (all of whose
-// sources are final), leaves its sums in `scratch` and takes a ticket of the pivot; the one that
+// The same, one level and direction per launch: the CTAs take the level's groups, from item `first` on, then
+// the late items of its pivots p0, ... (all of whose sources are final); each its sums in `scratch` and takes a ticket of the pivot; the one that
 // takes the last finishes the pivot with the arithmetic of k_flow.
 template <typename T, int NC, bool kFwd>
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(kFlowThreads, 1)
     k_stage(DevSym S, const T *__restrict__ slab, const T *__restrict__ wbuf, T *__restrict__ y, T *__restrict__ scratch,
-            int *__restrict__ tickets, const T *__restrict__ dinv, int64_t first, int64_t rows0, int nrhs, int max_m,
-            int stage)
+            int *__restrict__ tickets, int64_t p0, int64_t first, unsigned n_groups, int nrhs,
+            int max_m, int stage)
 {
     const FlowSmem<T> sm = flow_smem<T>(max_m, NC);
     const int tid = threadIdx.x;
-    const int64_t j = first + blockIdx.x, p = kFwd ? S.fwd_item_p[j] : S.bwd_item_p[j];
-    const FlowRow f = flow_row<kFwd>(S, S.piv[p]);
-    const int local = (int)(j - (kFwd ? S.fwdu_pref[p] : S.bwd_first[p])), m = f.m, E = m * nrhs;
-    const bool late = local == f.ng, has_w = kFwd && f.w >= 0;
+    const bool late = blockIdx.x >= n_groups;
+    const int64_t j = first + blockIdx.x;
+    const int64_t p = late ? p0 + (blockIdx.x - n_groups) : kFwd ? S.fwd_item_p[j] : S.bwd_item_p[j];
+    const FlowRow f = flow_row<kFwd, T>(S, S.piv[p]);
+    const int local = late ? f.ng : (int)(j - (kFwd ? S.fwdu_pref[p] : S.bwd_first[p])), m = f.m, E = m * nrhs;
+    const bool has_w = kFwd && f.w >= 0;
     const int i1 = late ? f.nb : f.ne - (f.ng - 1 - local) * kFlowGroup;
     const int i0 = late ? f.ne : max(0, i1 - kFlowGroup);
-    T *part = scratch + ((kFwd ? S.fwd_rows[p] : S.bwd_rows[p]) - rows0) * nrhs;
+    T *part = scratch + (kFwd ? S.fwd_rows[p] - S.fwd_rows[p0] : S.bwd_rows[p] - S.bwd_rows[p0]) * nrhs;
     T *yk = y + S.dof_off[f.k] * nrhs;
-    const int tpr = gemv_tpr<T>(m), rows = kThreads / tpr, q = tid & (tpr - 1);
+    const int tpr = gemv_tpr<T>(m), rows = kFlowThreads / tpr, q = tid & (tpr - 1);
     for (int ch = 0; ch < nrhs; ch += NC)
     {
         const int nc = min(NC, nrhs - ch);
@@ -515,11 +705,11 @@ __global__ void __launch_bounds__(kThreads, 2)
                     flow_load<kFwd>(g, S, f, slab, wbuf, i, c0, r0, tpr);
                     if (c0 == 0)
                     {
-                        for (int e = tid; e < g.K * nc; e += kThreads)
-                            sm.y[0][e / nc * NC + e % nc] = y[(g.src + e / nc) * nrhs + ch + e % nc];
+                        for (int e = tid; e < g.K * nc; e += kFlowThreads)
+                            sm.y[e / nc * NC + e % nc] = y[(g.src + e / nc) * nrhs + ch + e % nc];
                         __syncthreads();
                     }
-                    flow_add<T, NC>(a, g, sm.y[0], tpr);
+                    flow_add<T, NC>(a, g, sm.y, tpr);
                 }
             }
             flow_reduce<T, NC>(a, tpr);
@@ -535,11 +725,11 @@ __global__ void __launch_bounds__(kThreads, 2)
         return;
     FlowDiag<T> dg;
     if (kFwd)
-        flow_diag_load(dg, S, slab, dinv, f.k, m, sm.d, stage);
+        flow_diag_load(dg, S, slab, wbuf, f.k, m, tpr, sm.d, stage);
     for (int ch = 0; ch < nrhs; ch += NC)
     {
         const int nc = min(NC, nrhs - ch);
-        for (int e = tid; e < m * nc; e += kThreads)
+        for (int e = tid; e < m * nc; e += kFlowThreads)
         {
             const int64_t at = (int64_t)(e / nc) * nrhs + ch + e % nc;
             T v = yk[at];
@@ -556,12 +746,12 @@ __global__ void __launch_bounds__(kThreads, 2)
         }
         __syncthreads();
         if (kFwd)
-            flow_diag_solve<T, NC>(dg, S, slab, f.k, m, sm.acc, sm.part, sm.d, stage, nc);
-        for (int e = tid; e < m * nc; e += kThreads)
+            flow_diag_solve<T, NC>(dg, S, slab, wbuf, f.k, m, tpr, sm.acc, sm.y, sm.len, sm.d, stage, nc);
+        for (int e = tid; e < m * nc; e += kFlowThreads)
         {
             const int64_t at = (int64_t)(e / nc) * nrhs + ch + e % nc;
             T v = sm.acc[e / nc * NC + e % nc];
-            if (has_w)
+            if (has_w && f.nb > 0)
                 v -= __ldcg(part + (int64_t)f.ng * E + at);
             yk[at] = v;
         }
@@ -569,8 +759,8 @@ __global__ void __launch_bounds__(kThreads, 2)
     }
 }
 
-// W(k,s) = D_k^{-1} L(k,s) for the late blocks of the pivots that keep them, in FP64, once the factors are
-// final. grid.x: the W blocks, grid.y: their 64-column strips. Throughput only (one launch, off
+// X = D_k^{-1} and W(k,s) = D_k^{-1} L(k,s) for the late blocks of the pivots that keep them, in FP64, once
+// the factors are final. grid.x: the blocks (w_blk < 0: X), grid.y: their 64-column strips. Throughput only (one launch, off
 // the chain): 0.1 ms per 1,000 blocks of 64x64 on a B200.
 template <typename T>
 __global__ void __launch_bounds__(kFrontThreads, 2) k_late(DevSym S, const T *__restrict__ slab, T *__restrict__ wbuf)
@@ -579,8 +769,8 @@ __global__ void __launch_bounds__(kFrontThreads, 2) k_late(DevSym S, const T *__
     __shared__ int s_extreme;
     const int64_t blk = S.w_blk[blockIdx.x];
     const int64_t k = S.w_row[blockIdx.x];
-    const int m = S.size[k], K = S.size[S.cols[blk]], col0 = 64 * (int)blockIdx.y;
-    if (col0 >= K)
+    const int m = S.size[k], K = blk < 0 ? m : S.size[S.cols[blk]], col0 = 64 * (int)blockIdx.y;
+    if (col0 >= K || !flow_uses_w<T>(m))
         return;
     const int w = min(64, K - col0), nb = (w + 7) / 8, rows = front_rows(m), ldd = rows + 4;
     double *d = reinterpret_cast<double *>(smem_raw), *b = d + rows * ldd, *rpiv = b + rows * kLdStrip;
@@ -590,7 +780,12 @@ __global__ void __launch_bounds__(kFrontThreads, 2) k_late(DevSym S, const T *__
         s_extreme = 0;
     for (int c0 = 0; c0 < rows; c0 += 64)
         front_load(d + c0, ldd, gd + c0, m, m, m - c0, rows, min(64, rows - c0), warp, nw);
-    front_load(b, kLdStrip, slab + S.blk_off[blk] + col0, K, m, w, rows, 8 * nb, warp, nw);
+    if (blk >= 0)
+        front_load(b, kLdStrip, slab + S.blk_off[blk] + col0, K, m, w, rows, 8 * nb, warp, nw);
+    else
+        for (int r = warp; r < rows; r += nw)
+            for (int c = lane; c < 8 * nb; c += 32)
+                b[r * kLdStrip + c] = r == col0 + c;
     __syncthreads();
     if (tid < m)
     {

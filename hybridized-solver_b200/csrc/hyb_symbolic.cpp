@@ -374,20 +374,28 @@ int symbolic_build(int64_t n, const uint64_t *sizes, const uint64_t *row_ptr, co
         S.split_pref[p + 1] = S.split_pref[p] + n_lc + n_up;
         S.tc_pref[p + 1] = S.tc_pref[p] + n_lc * ((n_up + 1) / 2);
         // solve items: the early blocks of the row in groups, then one item for the late ones
-        const bool has_w = n_lr > 0 && S.size[k] >= kFlowLateMin && S.size[k] <= kFlowLateMax;
-        const int64_t ne = n_lr - std::min<int64_t>(n_lr, has_w ? kFlowLate : 1);
-        const int64_t nf = (ne + kFlowGroup - 1) / kFlowGroup + 1;
-        const int64_t nb = (std::max<int64_t>(0, n_up - kFlowLate) + kFlowGroup - 1) / kFlowGroup + 1;
+        const bool has_w = S.size[k] <= kFlowLateMax;
+        const int64_t ne = n_lr - std::min<int64_t>(n_lr, kFlowLate);
+        const int64_t nf = (ne + kFlowGroup - 1) / kFlowGroup;
+        const int64_t nb = (std::max<int64_t>(0, n_up - kFlowLate) + kFlowGroup - 1) / kFlowGroup;
         S.fwdu_pref[p + 1] = S.fwdu_pref[p] + nf;
         // partial-product spans padded to 4 values, so every pivot's partials start on a
         // 16-byte boundary in the staged (per-stage) and the dataflow (global) layouts alike
-        S.fwd_rows[p + 1] = S.fwd_rows[p] + ((n_lr > 0 ? nf : 0) * S.size[k] + 3) / 4 * 4;
-        S.bwd_rows[p + 1] = S.bwd_rows[p] + ((n_up > 0 ? nb : 0) * S.size[k] + 3) / 4 * 4;
+        S.fwd_rows[p + 1] = S.fwd_rows[p] + ((n_lr > 0 ? nf + 1 : 0) * S.size[k] + 3) / 4 * 4;
+        S.bwd_rows[p + 1] = S.bwd_rows[p] + ((n_up > 0 ? nb + 1 : 0) * S.size[k] + 3) / 4 * 4;
         fwd_span[p + 1] = fwd_span[p] + (n_lr * S.size[k] + 3) / 4 * 4;
         bwd_span[p + 1] = bwd_span[p] + (n_up * S.size[k] + 3) / 4 * 4;
         if (has_w)
         {
             S.w_off[k] = S.w_elems;
+            if (S.size[k] <= kFlowInvMax)
+            {
+                S.w_row.push_back((int32_t)k);
+                S.w_blk.push_back(-1);
+                S.w_out.push_back(S.w_elems);
+                S.w_elems += round_up((int64_t)S.size[k] * S.size[k], kFlowPad);
+                S.w_cols = std::max(S.w_cols, S.size[k]);
+            }
             for (int64_t j = S.row_ptr[k] + ne; j < S.diag_pos[k]; ++j)
             {
                 S.w_row.push_back((int32_t)k);
@@ -415,6 +423,7 @@ int symbolic_build(int64_t n, const uint64_t *sizes, const uint64_t *row_ptr, co
         for (int64_t j = S.fwdu_pref[p]; j < S.fwdu_pref[p + 1]; ++j)
             S.fwd_item_p[j] = (int32_t)p;
     S.bwd_item_p.clear();
+    S.bwd_slot.clear();
     S.bwd_first.assign(n, 0);
     S.bwd_lvl.assign(S.n_levels + 1, 0);
     for (int64_t l = S.n_levels - 1; l >= 0; --l)
@@ -425,7 +434,8 @@ int symbolic_build(int64_t n, const uint64_t *sizes, const uint64_t *row_ptr, co
             const int64_t k = S.piv[p];
             const int64_t n_up = S.row_ptr[k + 1] - S.diag_pos[k] - 1;
             S.bwd_first[p] = (int64_t)S.bwd_item_p.size();
-            const int64_t nb = (std::max<int64_t>(0, n_up - kFlowLate) + kFlowGroup - 1) / kFlowGroup + 1;
+            S.bwd_slot.push_back((int32_t)p);
+            const int64_t nb = (std::max<int64_t>(0, n_up - kFlowLate) + kFlowGroup - 1) / kFlowGroup;
             for (int64_t j = 0; j < nb; ++j)
                 S.bwd_item_p.push_back((int32_t)p);
         }
