@@ -529,26 +529,43 @@ bool fused_pivots(const Symbolic::LevelShape &sh)
     return sh.max_piv > 32 && sh.max_piv <= 64 && sh.max_up <= 128;
 }
 
-// Whether level l's 64-row pivots take the inverse-and-products path (HYB_OPTION_ROW_PIVOTS 2,
-// by default in the mixed form).
-template <typename T> bool inverse_pivots(const hyb_system *h, int64_t l)
-{
-    const Symbolic::LevelShape &sh = h->S.shape[l];
-    const int mode64 = h->row_pivots < 0 ? (std::is_same_v<T, float> ? 2 : 0) : h->row_pivots;
-    return std::is_same_v<T, float> && fused_pivots(sh) && sh.piv64 && mode64 == 2 && tc_level<T>(h, l) && h->d_dinv;
-}
+// Upper blocks of a pivot up to which a tensor-core level takes k_front. Its CTAs each factor the pivot, beside
+// the update's CTAs on the same SMs: with more of them the one CTA of k_piv64_inv and its
+// products are sooner done. Mixed factorizations at 40x40 p=8 62 ms (k_front) against 70, at 48x48
+// 101 against 99, at 64x64 205 against 187.
+constexpr int64_t kFrontTcMax = 44;
 
-// Whether a level's pivots take k_front: all of up to 128 rows, except where an option asks for
-// one of the 64-row kernels by name (HYB_OPTION_ROW_PIVOTS, HYB_OPTION_PIVOT_LU_ONCE).
-bool front_pivots(const hyb_system *h, const Symbolic::LevelShape &sh)
+// Whether level l's pivots take k_front: all of up to 128 rows, except where an option asks for
+// one of the 64-row kernels by name (HYB_OPTION_ROW_PIVOTS, HYB_OPTION_PIVOT_LU_ONCE) and on
+// tensor-core levels with many upper blocks.
+template <typename T> bool front_pivots(const hyb_system *h, int64_t l)
 {
+    const Symbolic &S = h->S;
+    const Symbolic::LevelShape &sh = S.shape[l];
     if (sh.max_piv > hyb::kFrontMax)
         return false;
-    return !fused_pivots(sh) || (h->lu_once < 0 && h->row_pivots < 0);
+    if (!fused_pivots(sh))
+        return true;
+    const int64_t p0 = S.lvl_ptr[l], p1 = S.lvl_ptr[l + 1];
+    return h->lu_once < 0 && h->row_pivots < 0 &&
+           !(tc_level<T>(h, l) && S.trsm_pref[p1] - S.trsm_pref[p0] > kFrontTcMax * (p1 - p0));
 }
 
-// LU and row solves of level l's pivots by k_front.
-template <typename T> int enqueue_front(hyb_system *h, T *slab, int64_t l, cudaStream_t st, uint64_t &launches)
+// Whether level l's pivot can take the update of its row and column by level lp's on the way: k_front, single
+// pivots, every block concerned at most 64 wide.
+template <typename T> bool front_takes(const hyb_system *h, int64_t lp, int64_t l)
+{
+    const Symbolic &S = h->S;
+    const Symbolic::LevelShape &a = S.shape[lp], &b = S.shape[l];
+    auto single = [&](int64_t x) { return S.lvl_ptr[x + 1] - S.lvl_ptr[x] == 1; };
+    return single(lp) && single(l) && front_pivots<T>(h, l) &&
+           std::max({a.max_piv, a.max_row, a.max_up, b.max_piv, b.max_row, b.max_up}) <= hyb::kPrevMax;
+}
+
+// LU and row solves of level l's pivots by k_front; prev >= 0: with the update of their row and column by
+// level prev's pivot. Tensor-core levels get their operands (splits, target table) from it.
+template <typename T>
+int enqueue_front(hyb_system *h, T *slab, int64_t l, cudaStream_t st, uint64_t &launches, int64_t prev = -1)
 {
     const Symbolic &S = h->S;
     const int64_t p0 = S.lvl_ptr[l], p1 = S.lvl_ptr[l + 1];
@@ -560,12 +577,55 @@ template <typename T> int enqueue_front(hyb_system *h, T *slab, int64_t l, cudaS
     int strip = 64;
     while (strip > 16 && units * ((sh.max_up + strip / 2 - 1) / (strip / 2)) <= sm_count())
         strip /= 2;
-    const dim3 grid((unsigned)units, (unsigned)std::max(1, (sh.max_up + strip - 1) / strip));
-    hyb::k_front<T><<<grid, hyb::kFrontThreads, hyb::front_smem(sh.max_piv), st>>>(h->ds, slab, p0, p1, h->d_lu_tickets,
-                                                                                 h->d_status, glim, strip);
+    const bool tc = tc_level<T>(h, l);
+    if (tc || prev >= 0)
+        strip = std::min(strip, 32); // room beside an update CTA (front_smem)
+    hyb::FrontOne one;
+    if (p1 - p0 == 1)
+    {
+        one.k = S.piv[p0];
+        one.m = S.size[one.k];
+        one.dpos = S.diag_pos[one.k];
+        one.end = S.row_ptr[one.k + 1];
+        one.doff = S.blk_off[one.dpos];
+    }
+    if (prev >= 0)
+    {
+        one.kp = S.piv[S.lvl_ptr[prev]];
+        one.Kp = S.size[one.kp];
+        one.ip = S.shape[prev].la_i0;
+        one.jp = S.shape[prev].la_j0;
+        one.u0 = S.diag_pos[one.kp] + 1;
+        one.uend = S.row_ptr[one.kp + 1];
+        one.l0 = S.lcol_ptr[one.kp];
+        one.lend = S.lcol_ptr[one.kp + 1];
+        if (one.ip >= 0)
+            one.loff = S.blk_off[S.lcol_blk[one.l0 + one.ip]];
+        if (one.jp >= 0)
+            one.udoff = S.blk_off[one.u0 + one.jp];
+    }
+    const int64_t lower = (S.split_pref[p1] - S.trsm_pref[p1]) - (S.split_pref[p0] - S.trsm_pref[p0]);
+    const dim3 grid((unsigned)(units + (tc || one.jp >= 0 ? lower : 0)),
+                    (unsigned)std::max(1, (sh.max_up + strip - 1) / strip));
+    // column units hold a 64-row strip and an update's operands whatever the pivot's size
+    int smem = hyb::front_smem(sh.max_piv, strip, prev >= 0);
+    if (tc || prev >= 0)
+        smem = std::max(smem, hyb::front_column_smem());
+    hyb::k_front<T><<<grid, hyb::kFrontThreads, smem, st>>>(
+        h->ds, slab, p0, p1, h->d_lu_tickets, h->d_status, glim, strip, (unsigned)units, one,
+        tc ? level_ops(h, l) : nullptr, tc ? level_tgt(h, l) : nullptr);
     ++launches;
     HYB_LAUNCHED("k_front", l);
-    return enqueue_split<T>(h, slab, l, st, launches);
+    return HYB_SUCCESS;
+}
+
+// Whether level l's 64-row pivots take the inverse-and-products path (HYB_OPTION_ROW_PIVOTS 2, or -1 where
+// k_front is the slower one).
+template <typename T> bool inverse_pivots(const hyb_system *h, int64_t l)
+{
+    const Symbolic::LevelShape &sh = h->S.shape[l];
+    return std::is_same_v<T, float> && fused_pivots(sh) && sh.piv64 && tc_level<T>(h, l) && h->d_dinv &&
+           (h->row_pivots == 2 || (h->row_pivots < 0 && !front_pivots<T>(h, l)));
 }
 
 // With pair_first (level l's pivot is the first of a pair on the inverse-and-products path),
@@ -573,9 +633,10 @@ template <typename T> int enqueue_front(hyb_system *h, T *slab, int64_t l, cudaS
 // kernel too; the caller then issues no separate update for it.
 // With second_done (level l's pivot is the second of such a pair), its LU and inverse were
 // formed by the first pivot's products launch: only its products (and splits) remain.
+// With prev >= 0 (front_takes) the update of the pivot's row and column by level prev's is included.
 template <typename T>
 int enqueue_pivots(hyb_system *h, T *slab, int64_t l, cudaStream_t st, uint64_t &launches, bool pair_first = false,
-                   bool second_done = false)
+                   bool second_done = false, int64_t prev = -1)
 {
     const Symbolic &S = h->S;
     const DevSym &ds = h->ds;
@@ -584,12 +645,12 @@ int enqueue_pivots(hyb_system *h, T *slab, int64_t l, cudaStream_t st, uint64_t 
     const Symbolic::LevelShape &sh = S.shape[l];
     // growth check and FP64 fallback of the mixed form (0: off, and always for FP64 factors)
     const float glim = std::is_same_v<T, float> && h->d_hg ? h->growth_limit : 0.0f;
-    // 64-row pivots (HYB_OPTION_ROW_PIVOTS): the mixed form by default factors each pivot
-    // once and takes its upper blocks as products with the inverse (2); 1 is the blocked
-    // substitution kernel (bit-identical to the 256-thread kernels); the FP64 form keeps the
-    // 256-thread kernels by default, since the blocked kernel's 115 KB of FP64 shared
-    // memory displaces update CTAs (measured at 96x96 p=8: 2,229 against 2,138 ms)
-    const int mode64 = h->row_pivots < 0 ? (std::is_same_v<T, float> ? 2 : 0) : h->row_pivots;
+    // 64-row pivots where HYB_OPTION_ROW_PIVOTS asks for a kernel: factored once with the upper blocks as
+    // products with the inverse (2), or the blocked substitution kernel (1; bit-identical to the
+    // 256-thread kernels)
+    const int mode64 = std::max(0, h->row_pivots);
+    if (front_pivots<T>(h, l))
+        return enqueue_front<T>(h, slab, l, st, launches, prev);
     if constexpr (std::is_same_v<T, float>)
     {
         if (inverse_pivots<T>(h, l))
@@ -667,7 +728,7 @@ int enqueue_pivots(hyb_system *h, T *slab, int64_t l, cudaStream_t st, uint64_t 
         HYB_LAUNCHED("k_piv64", l);
         return HYB_SUCCESS;
     }
-    if (fused_pivots(sh) && !front_pivots(h, sh))
+    if (fused_pivots(sh))
     {
         // fused: diagonal LU (padded to 64x64) and the solves of the pivot rows' upper blocks;
         // pivots of up to 32 rows stay on the generic kernels, whose serial steps are short
@@ -714,8 +775,6 @@ int enqueue_pivots(hyb_system *h, T *slab, int64_t l, cudaStream_t st, uint64_t 
         HYB_LAUNCHED("k_lu_trsm64", l);
         return enqueue_split<T>(h, slab, l, st, launches);
     }
-    if (front_pivots(h, sh))
-        return enqueue_front<T>(h, slab, l, st, launches);
     const int lu_bytes = lu_smem_bytes<T>(sh.max_piv);
     int *hg = glim > 0 ? h->d_hg : nullptr;
     if (lu_bytes <= optin)
@@ -763,7 +822,7 @@ template <typename T> int enqueue_late(hyb_system *h, T *slab, uint64_t &launche
     for (int32_t k : S.w_row)
         m = std::max(m, S.size[k]);
     const dim3 grid((unsigned)S.w_blk.size(), (unsigned)((S.w_cols + 63) / 64));
-    hyb::k_late<T><<<grid, hyb::kFrontThreads, hyb::front_smem(m), h->stream>>>(h->ds, slab, late_blocks<T>(h));
+    hyb::k_late<T><<<grid, hyb::kFrontThreads, hyb::front_smem(m, 64), h->stream>>>(h->ds, slab, late_blocks<T>(h));
     ++launches;
     HYB_LAUNCHED("k_late", S.n_levels - 1);
     return HYB_SUCCESS;
@@ -999,15 +1058,18 @@ template <typename T> bool pair_unit(const hyb_system *h, int64_t l)
 // split. A pair (a, b): a's, then a's update of b's row and column -- a few hundred target
 // blocks in FP32 on the CUDA cores, in CTAs small enough to run beside a tensor-core pass --
 // then b's.
-template <typename T> int enqueue_unit_pivots(hyb_system *h, T *slab, int64_t l, cudaStream_t st, uint64_t &launches)
+template <typename T>
+int enqueue_unit_pivots(hyb_system *h, T *slab, int64_t l, cudaStream_t st, uint64_t &launches, int64_t prev = -1)
 {
     const bool pair = pair_unit<T>(h, l);
     const bool fold = pair && h->pair_passes == 1 && inverse_pivots<T>(h, l) && inverse_pivots<T>(h, l + 1) &&
                       h->S.shape[l].la_i0 >= 0 && h->S.shape[l].la_j0 >= 0;
-    int rc = enqueue_pivots<T>(h, slab, l, st, launches, fold);
+    int rc = enqueue_pivots<T>(h, slab, l, st, launches, fold, false, prev);
     if (rc != HYB_SUCCESS || !pair)
         return rc;
     const Symbolic::LevelShape &sh = h->S.shape[l];
+    if (h->pair_passes == 1 && front_takes<T>(h, l, l + 1))
+        return enqueue_pivots<T>(h, slab, l + 1, st, launches, false, false, l);
     if (!fold && (rc = enqueue_generic_update<T>(h, slab, l, st, 1, sh.la_prio_units, UPD_TILE32, launches)) !=
                      HYB_SUCCESS)
         return rc;
@@ -1061,7 +1123,7 @@ template <typename T> int enqueue_factor(hyb_system *h, T *slab, uint64_t &launc
     int64_t nl = 1;
     // the pivot work of the unit at level lu on stream s, bracketed by events on every
     // profile-th unit
-    auto unit_pivots = [&](int64_t lu, cudaStream_t s) -> int {
+    auto unit_pivots = [&](int64_t lu, cudaStream_t s, int64_t prev = -1) -> int {
         const bool tp = h->profile > 0 && h->prof_piv_units++ % h->profile == 0;
         if (tp)
         {
@@ -1073,7 +1135,7 @@ template <typename T> int enqueue_factor(hyb_system *h, T *slab, uint64_t &launc
             h->prof_piv_levels.push_back(pair_unit<T>(h, lu) ? 2 : 1);
             HYB_CUDA(cudaEventRecordWithFlags(e0, s, cudaEventRecordExternal));
         }
-        const int r = enqueue_unit_pivots<T>(h, slab, lu, s, launches);
+        const int r = enqueue_unit_pivots<T>(h, slab, lu, s, launches, prev);
         if (r == HYB_SUCCESS && tp)
             HYB_CUDA(cudaEventRecordWithFlags(h->prof_piv_ev.back(), s, cudaEventRecordExternal));
         return r;
@@ -1118,11 +1180,14 @@ template <typename T> int enqueue_factor(hyb_system *h, T *slab, uint64_t &launc
         };
         if (lookahead)
         {
-            if ((rc = update(1)) != HYB_SUCCESS)
+            // FP64: the next pivot's kernel updates its row and column itself. (FP32 updates are rounded by
+            // the kernel that makes them, and lookahead does not change the factors.)
+            const bool taken = std::is_same_v<T, double> && !pair && front_takes<T>(h, l, next);
+            if (!taken && (rc = update(1)) != HYB_SUCCESS)
                 return rc;
             HYB_CUDA(cudaEventRecord(h->ev_prio, st));
             HYB_CUDA(cudaStreamWaitEvent(st2, h->ev_prio, 0));
-            if ((rc = unit_pivots(next, st2)) != HYB_SUCCESS)
+            if ((rc = unit_pivots(next, st2, taken ? l : -1)) != HYB_SUCCESS)
                 return rc;
             HYB_CUDA(cudaEventRecord(h->ev_piv, st2));
             if ((rc = update(2)) != HYB_SUCCESS)
@@ -2414,8 +2479,8 @@ HYB_API int hyb_decompose(hyb_system *h, int precision, hyb_decompose_info *info
             allow_smem(hyb::k_lu<float, true>, optin),
             allow_smem(hyb::k_trsm<double, true>, optin),
             allow_smem(hyb::k_trsm<float, true>, optin),
-            allow_smem(hyb::k_late<double>, hyb::front_smem(hyb::kFlowLateMax)),
-            allow_smem(hyb::k_late<float>, hyb::front_smem(hyb::kFlowLateMax)),
+            allow_smem(hyb::k_late<double>, hyb::front_smem(hyb::kFlowLateMax, 64)),
+            allow_smem(hyb::k_late<float>, hyb::front_smem(hyb::kFlowLateMax, 64)),
             allow_smem(hyb::k_update64_f64<0>, hyb::kUpd64Smem),
             allow_smem(hyb::k_update64_f64<1>, hyb::kUpd64Smem),
             allow_smem(hyb::k_update64_f64<2>, hyb::kUpd64Smem),
@@ -2431,8 +2496,8 @@ HYB_API int hyb_decompose(hyb_system *h, int precision, hyb_decompose_info *info
             allow_smem(hyb::k_piv64_inv, hyb::kInvSmem),
             allow_smem(hyb::k_strips64_inv, hyb::kInvSmem),
             allow_smem(hyb::k_split64, 0),
-            allow_smem(hyb::k_front<double>, hyb::front_smem(hyb::kFrontMax)),
-            allow_smem(hyb::k_front<float>, hyb::front_smem(hyb::kFrontMax)),
+            allow_smem(hyb::k_front<double>, hyb::front_smem(hyb::kFrontMax, 64)),
+            allow_smem(hyb::k_front<float>, hyb::front_smem(hyb::kFrontMax, 64)),
             allow_smem(hyb::k_update<double>, 0),
             allow_smem(hyb::k_update<float>, 0),
             allow_smem(hyb::k_update32<double>, 0),
@@ -2511,10 +2576,13 @@ HYB_API int hyb_decompose(hyb_system *h, int precision, hyb_decompose_info *info
         {
             HYB_CUDA(cudaMalloc(&h->d_f32, slab * sizeof(float)));
             HYB_CUDA(cudaMalloc(&h->d_w32, std::max<int64_t>(1, S.w_elems) * sizeof(float)));
-            if (S.n_inv > 0)
-                HYB_CUDA(cudaMalloc(&h->d_dinv, (size_t)S.n_inv * 4096 * sizeof(float)));
             h->g_factor[1].reset();
             h->g_solve.clear();
+        }
+        if (h->row_pivots != 0 && h->row_pivots != 1 && !h->d_dinv && S.n_inv > 0)
+        {
+            HYB_CUDA(cudaMalloc(&h->d_dinv, (size_t)S.n_inv * 4096 * sizeof(float)));
+            h->g_factor[1].reset();
         }
         if (!h->d_hg)
         {

@@ -18,15 +18,17 @@
 // The factorization of FP32 factors (T = float) runs in FP64 as well and rounds once, when
 // the results are stored: an FP32 reciprocal is no shorter (77 cycles), so FP32 would save no
 // time on the chain and would need a second, FP64 path for pivots with growth.
-// Measured on a B200 in one CTA, in SM cycles: a 64x64 block 17.5k for the LU with a strip's
-// forward part and 10.7k for its backward part (16 columns; 21k and 14k with 64), where the
-// 256-thread kernels took 69k for the FP64 LU alone and 38k for a strip of 64; 16x16 3.7k and
-// 2.5k. Factorization time of whole meshes, before and after: 25x25 p=6 53.0 to 16.2 ms, 24x24
-// p=8 44.5 to 21.3 ms, 32x32 of orders 2..10 123 to 55 ms, 16x16 p=4 5.6 to 2.8 ms. The factors
-// of both are the same but for the rounding of 33- to 64-row pivots.
+// Measured on a B200 in one CTA, in SM cycles: a 64x64 block 18k for the LU with a strip's
+// forward part (23k to 25k beside CTAs of an update on the same SM) and 5.5k for its backward part (16 columns),
+// where the 256-thread kernels took 69k for the FP64 LU alone and 38k for a strip of 64; 16x16
+// 3.7k and 2.5k; the update by the pivot before, taken on the way, 13k for 64 rows. Factorization time of
+// whole meshes -- with the 256-thread kernels, with this kernel alone, and with the update inside it:
+// 25x25 p=6 53.0, 16.2 and 13.3 ms, 24x24 p=8 44.5, 21.3 and 20.0 ms, 16x16 p=4 5.6, 2.8 and 2.2 ms;
+// mixed 31x31 p=8 41.1 and 34.5 ms (pairs of pivots). The factors are the same but for the
+// rounding of pivots of more than 16 rows.
 #pragma once
 
-#include "hyb_kernels.cuh"
+#include "hyb_umma.cuh"
 
 namespace hyb
 {
@@ -34,7 +36,13 @@ namespace hyb
 constexpr int kFrontThreads = 256;
 constexpr int kFrontMax = 128; // largest pivot
 constexpr int kPanel = 8;
-constexpr int kLdStrip = 68; // row stride of the strip: 4 mod 16 doubles, conflict-free DMMA operands
+constexpr int kLdUinv = 12; // row stride of the inverses of U's diagonal blocks: conflict-free DMMA operands
+constexpr int kExactMax = 16; // largest pivot whose strips are substituted to the bit
+
+// Contraction per step of the update by the pivot before, and the row stride of its left operand.
+constexpr int kPrevK = 16;
+constexpr int kLdPrev = kPrevK + 4; // conflict-free left operands
+constexpr int kPrevMax = 64;        // largest blocks that take it
 
 // The block and the strip are held with their rows rounded up to 16.
 __host__ __device__ constexpr int front_rows(int m)
@@ -42,11 +50,28 @@ __host__ __device__ constexpr int front_rows(int m)
     return (m + 15) / 16 * 16;
 }
 
-// Dynamic shared memory for pivots of up to m rows: the block (row stride 4 mod 16 doubles), the strip,
-// the pivots' reciprocals and eight pivot rows of a panel.
-__host__ __device__ constexpr int front_smem(int m)
+// Row stride of a strip of up to w columns (a multiple of 16): 4 mod 16 doubles.
+__host__ __device__ constexpr int front_ldb(int w)
 {
-    return (front_rows(m) * (front_rows(m) + 4) + front_rows(m) * kLdStrip + front_rows(m) + kPanel * kPanel) * 8;
+    return w + 4;
+}
+
+// Dynamic shared memory for pivots of up to m rows and strips of w columns: the block (row stride 4 mod 16
+// doubles), the strip, the pivots' reciprocals, eight pivot rows of a panel and the inverses of U's
+// 8x8 diagonal blocks; with `prev` the operands of a step of the update by the pivot before. 83 KB for
+// 64 rows and 32 columns with it: beside a CTA of the mixed form's update (129 KB) an SM has room
+// for one.
+__host__ __device__ constexpr int front_smem(int m, int w, bool prev = false)
+{
+    return (front_rows(m) * (front_rows(m) + 4) + front_rows(m) * front_ldb(w) + front_rows(m) + kPanel * kPanel +
+            front_rows(m) * kLdUinv + (prev ? kPrevMax * kLdPrev + kPrevK * (front_ldb(kPrevMax) + front_ldb(w)) : 0)) *
+           8;
+}
+
+// The same for the column units: a 64 x 64 strip and a step's operands.
+__host__ __device__ constexpr int front_column_smem()
+{
+    return (kPrevMax * front_ldb(kPrevMax) + kPrevMax * kLdPrev + 2 * kPrevK * front_ldb(kPrevMax)) * 8;
 }
 
 // 1 / p to within an ulp for a pivot that is not extreme: the hardware's approximation (PTX
@@ -199,46 +224,53 @@ __device__ __forceinline__ void front_panel(double *d, int ld, int r0, int rows,
             *reinterpret_cast<double2 *>(rpiv + r0 + c) = make_double2(rp[c], rp[c + 1]);
 }
 
-// c -= a b on 8x8 tiles in shared memory with a contraction of eight, by one warp: the rows row0,
-// row0 + 8, ... < rows of the column tile at c (row stride ldc), a (row stride lda) the eight
-// columns of the same rows, b (row stride ldb) the eight rows of the column tile, the first kw of
-// which count (what lies beyond the block's edge may be anything).
-// kBatch tiles are loaded before the first is stored: their latencies overlap. With kDown the
-// contraction runs from the last of the eight down, the order of a backward substitution.
-template <int kBatch, bool kDown = false>
-__device__ __forceinline__ void front_tiles(double *c, int ldc, const double *a, int lda, const double *b, int ldb,
-                                            int row0, int rows, int kw = kPanel)
+// kBatch 8x8 tiles, one below the other: c -= a b with a contraction of eight, by one warp. The tiles are
+// loaded before the first is stored, so that their latencies overlap.
+template <int kBatch, bool kDown>
+__device__ __forceinline__ void front_batch(double *pc, int ldc, const double *pa, int lda, double b0, double b1, int k0,
+                                            int k1, int kw)
+{
+    double2 v[kBatch];
+    double a0[kBatch], a1[kBatch];
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i)
+    {
+        v[i] = *reinterpret_cast<double2 *>(pc + 8 * i * ldc);
+        a0[i] = k0 < kw ? -pa[8 * i * lda + k0] : 0.0;
+        a1[i] = k1 < kw ? -pa[8 * i * lda + k1] : 0.0;
+    }
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i)
+        dmma_8x8x4(v[i].x, v[i].y, a0[i], b0);
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i)
+        dmma_8x8x4(v[i].x, v[i].y, a1[i], b1);
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i)
+        *reinterpret_cast<double2 *>(pc + 8 * i * ldc) = v[i];
+}
+
+// c -= a b for the tiles t0 .. t1 - 1 (of eight rows) of a column tile in shared memory, by one warp: c (row
+// stride ldc) and a (row stride lda; eight columns) from their row 0, b (row stride ldb) the eight
+// rows of the column tile, the first kw of which count (what lies beyond the block's edge may be
+// anything). With kDown the contraction runs from the last of the eight down, the order of a
+// backward substitution. Whole batches without a test per tile: with one, the compiler put a
+// branch around every product, and a call took 1,000 cycles instead of 200.
+template <bool kDown = false>
+__device__ __forceinline__ void front_tiles(double *c, int ldc, const double *a, int lda, const double *b, int ldb, int t0,
+                                            int t1, int kw = kPanel)
 {
     const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
     const int k0 = kDown ? 7 - q : q, k1 = kDown ? 3 - q : 4 + q;
     const double b0 = k0 < kw ? b[k0 * ldb + g] : 0.0, b1 = k1 < kw ? b[k1 * ldb + g] : 0.0;
-    double *pc = c + (row0 + g) * ldc + 2 * q;
-    const double *pa = a + (row0 + g) * lda;
+    double *pc = c + (8 * t0 + g) * ldc + 2 * q;
+    const double *pa = a + (8 * t0 + g) * lda;
 #pragma unroll 1
-    for (int r = row0; r < rows; r += 8 * kBatch, pc += 8 * kBatch * ldc, pa += 8 * kBatch * lda)
-    {
-        double2 v[kBatch];
-        double a0[kBatch], a1[kBatch];
-#pragma unroll
-        for (int i = 0; i < kBatch; ++i)
-            if (i == 0 || r + 8 * i < rows)
-            {
-                v[i] = *reinterpret_cast<double2 *>(pc + 8 * i * ldc);
-                a0[i] = pa[8 * i * lda + k0];
-                a1[i] = pa[8 * i * lda + k1];
-            }
-#pragma unroll
-        for (int i = 0; i < kBatch; ++i)
-            if (i == 0 || r + 8 * i < rows)
-            {
-                dmma_8x8x4(v[i].x, v[i].y, k0 < kw ? -a0[i] : 0.0, b0);
-                dmma_8x8x4(v[i].x, v[i].y, k1 < kw ? -a1[i] : 0.0, b1);
-            }
-#pragma unroll
-        for (int i = 0; i < kBatch; ++i)
-            if (i == 0 || r + 8 * i < rows)
-                *reinterpret_cast<double2 *>(pc + 8 * i * ldc) = v[i];
-    }
+    for (; t0 + 4 <= t1; t0 += 4, pc += 32 * ldc, pa += 32 * lda)
+        front_batch<4, kDown>(pc, ldc, pa, lda, b0, b1, k0, k1, kw);
+#pragma unroll 1
+    for (; t0 < t1; ++t0, pc += 8 * ldc, pa += 8 * lda)
+        front_batch<1, kDown>(pc, ldc, pa, lda, b0, b1, k0, k1, kw);
 }
 
 // Eight rows of one column (stride ld) <- L^{-1} of them, L the unit lower block at d (row stride ldd).
@@ -293,12 +325,36 @@ __device__ __noinline__ void front_backward_divide(const double *d, int ldd, dou
     front_backward<true>(d, ldd, nullptr, col, ld, w);
 }
 
+// Column c (0 .. 7) of the inverse of the upper 8x8 block at d (row stride ldd; w rows of it in use), by one
+// thread, into out (row stride kLdUinv); rpiv: its pivots' reciprocals.
+__device__ __forceinline__ void front_uinv(const double *d, int ldd, const double *rpiv, int w, int c, double *out)
+{
+    double x[kPanel];
+#pragma unroll
+    for (int i = 0; i < kPanel; ++i)
+        x[i] = i == c && c < w ? 1.0 : 0.0;
+#pragma unroll
+    for (int k = kPanel - 1; k >= 0; --k)
+    {
+        if (k >= w)
+            continue;
+        x[k] = front_quotient(x[k], d[k * ldd + k], rpiv[k]);
+#pragma unroll
+        for (int i = 0; i < k; ++i)
+            x[i] = fma(-d[i * ldd + k], x[k], x[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < kPanel; ++i)
+        out[i * kLdUinv + c] = x[i];
+}
+
 // Loads rows x cols values of a row-major block (row stride lds) into shared memory (row stride ld),
-// as doubles, zero up to prows x pcols (pcols at most 64); warp `warp` of nw. Sixteen values per
+// as doubles, continued up to prows x pcols (pcols at most 64) by zeros or, with diag >= 0, the block's
+// columns being those from diag on of a square one, by the identity; warp `warp` of nw. Sixteen values per
 // lane are in flight at once. Returns the largest magnitude.
 template <typename T>
 __device__ __forceinline__ double front_load(double *dst, int ld, const T *src, int lds, int rows, int cols, int prows,
-                                             int pcols, int warp, int nw)
+                                             int pcols, int warp, int nw, int diag = -1)
 {
     const int lane = threadIdx.x & 31;
     double amax = 0;
@@ -320,7 +376,7 @@ __device__ __forceinline__ double front_load(double *dst, int ld, const T *src, 
             {
                 const int r = r0 + i * nw, c = lane + 32 * h;
                 if (r < prows && c < pcols)
-                    dst[r * ld + c] = v[i][h];
+                    dst[r * ld + c] = diag >= 0 && r >= rows && r == diag + c ? 1.0 : v[i][h];
                 amax = fmax(amax, fabs(v[i][h]));
             }
     }
@@ -329,14 +385,16 @@ __device__ __forceinline__ double front_load(double *dst, int ld, const T *src, 
 
 // LU of the m x m block d in shared memory (row stride ldd, continued by the identity up to the
 // next multiple of 16) and, as further columns, b <- L^{-1} b for the nb tiles of eight columns of
-// the strip b. `load_strip` (called by the warps other than the first, with their number among
-// them and their count) fills b before it is first read; it runs beside the first panel.
+// the strip b (row stride ldb). `load_strip` (called by the warps other than the panel's, with their
+// number among them and their count) fills b before it is first read; it runs beside the first
+// panel. uinv (or null): the inverses of U's diagonal blocks.
 template <typename F>
-__device__ __forceinline__ void front_factor(double *d, int ldd, int m, double *b, int nb, double *rpiv, double *ubuf,
-                                             int *flags, F load_strip)
+__device__ __forceinline__ void front_factor(double *d, int ldd, int m, double *b, int ldb, int nb, double *rpiv,
+                                             double *ubuf, int *flags, double *uinv, F load_strip)
 {
     const int tid = threadIdx.x, warp = tid >> 5, nw = kFrontThreads / 32;
     const int rows = (m + kPanel - 1) / kPanel * kPanel;
+#pragma unroll 1
     for (int r0 = 0; r0 < rows; r0 += kPanel)
     {
         const int r1 = r0 + kPanel, w = min(kPanel, m - r0);
@@ -351,14 +409,17 @@ __device__ __forceinline__ void front_factor(double *d, int ldd, int m, double *
         }
         else
         {
-            // the panel before on the columns beyond this one, in units of a column tile and up to four rows of tiles
-            const int nd = (rows - r1) / 8, k0 = r0 - kPanel, nc = nd + nb;
-            for (int t = warp - np; t < nc * ((rows - r0 + 31) / 32); t += nw - np)
+            // the panel before's upper block, inverted for the backward substitution
+            const int nd = (rows - r1) / 8, k0 = r0 - kPanel, n = (rows - r0) / 8;
+            if (uinv && warp == nw - 1 && (tid & 31) < kPanel)
+                front_uinv(d + k0 * ldd + k0, ldd, rpiv + k0, kPanel, tid & 31, uinv + k0 * kLdUinv);
+            // the panel before on the columns beyond this one, in halves of a column tile
+            for (int t = warp - np; t < 2 * (nd + nb); t += nw - np)
             {
-                const int i = t % nc, row = r0 + t / nc * 32;
+                const int i = t >> 1, lo = t & 1 ? n >> 1 : 0, hi = t & 1 ? n : n >> 1;
                 double *c = i < nd ? d + r1 + 8 * i : b + 8 * (i - nd);
-                const int ldc = i < nd ? ldd : kLdStrip;
-                front_tiles<4>(c, ldc, d + k0, ldd, c + k0 * ldc, ldc, row, min(row + 32, rows));
+                const int ldc = i < nd ? ldd : ldb;
+                front_tiles(c + r0 * ldc, ldc, d + r0 * ldd + k0, ldd, c + k0 * ldc, ldc, lo, hi);
             }
         }
         __syncthreads();
@@ -366,96 +427,367 @@ __device__ __forceinline__ void front_factor(double *d, int ldd, int m, double *
         const int nd = rows - r1;
         for (int t = tid; t < nd + 8 * nb; t += kFrontThreads)
         {
-            const int ldc = t < nd ? ldd : kLdStrip;
-            front_forward(d + r0 * ldd + r0, ldd, t < nd ? d + r0 * ldd + r1 + t : b + r0 * kLdStrip + t - nd, ldc);
+            const int ldc = t < nd ? ldd : ldb;
+            front_forward(d + r0 * ldd + r0, ldd, t < nd ? d + r0 * ldd + r1 + t : b + r0 * ldb + t - nd, ldc);
         }
         __syncthreads();
         // the next panel's columns, so that it can start
         if (nd > 0)
         {
-            for (int row = r1 + 8 * warp; row < rows; row += 8 * nw)
-                front_tiles<1>(d + r1, ldd, d + r0, ldd, d + r0 * ldd + r1, ldd, row, row + 8);
+            for (int t = warp; 8 * t < nd; t += nw)
+                front_tiles(d + r1 * ldd + r1, ldd, d + r1 * ldd + r0, ldd, d + r0 * ldd + r1, ldd, t, t + 1);
             __syncthreads();
+        }
+        else if (uinv && tid < kPanel)
+        {
+            front_uinv(d + r0 * ldd + r0, ldd, rpiv + r0, w, tid, uinv + r0 * kLdUinv);
         }
     }
 }
 
-// b <- U^{-1} b for the strip, U the upper factor in d. Two warps solve eight rows of the strip's
-// columns while the others apply the eight rows below to the rows above them.
-__device__ __forceinline__ void front_back(const double *d, int ldd, int m, double *b, int nb, const double *rpiv,
+// b <- U^{-1} b for the strip by products: eight rows at a time with the inverse of U's diagonal block (uinv),
+// then the rows above in quarters of a column tile. The 8x8 inverses are as close to substitution
+// as U's blocks are well conditioned; a substitution spends 430 cycles on eight rows, the product 200.
+__device__ __forceinline__ void front_back_products(const double *d, int ldd, int m, double *b, int ldb, int nb,
+                                                    const double *uinv)
+{
+    const int tid = threadIdx.x, warp = tid >> 5, nw = kFrontThreads / 32, lane = tid & 31, g = lane >> 2, q = lane & 3;
+#pragma unroll 1
+    for (int r0 = (m - 1) / kPanel * kPanel; r0 >= 0; r0 -= kPanel)
+    {
+        const int w = min(kPanel, m - r0);
+        __syncthreads(); // the rows r0 .. are up to date, and uinv is written
+        if (warp < nb)
+        {
+            double2 x = make_double2(0, 0);
+            double *c = b + r0 * ldb + 8 * warp;
+            const double *a = uinv + (r0 + g) * kLdUinv;
+            dmma_8x8x4(x.x, x.y, a[q], q < w ? c[q * ldb + g] : 0.0);
+            dmma_8x8x4(x.x, x.y, a[4 + q], 4 + q < w ? c[(4 + q) * ldb + g] : 0.0);
+            __syncwarp();
+            *reinterpret_cast<double2 *>(c + g * ldb + 2 * q) = x;
+        }
+        if (r0 == 0)
+            break;
+        __syncthreads();
+        const int n = r0 / 8;
+        for (int t = warp; t < 4 * nb; t += nw)
+        {
+            const int col = t >> 2, part = t & 3;
+            front_tiles(b + 8 * col, ldb, d + r0, ldd, b + r0 * ldb + 8 * col, ldb, n * part >> 2, n * (part + 1) >> 2, w);
+        }
+    }
+    __syncthreads();
+}
+
+// b <- U^{-1} b for the strip, U the upper factor in d, by substitution. Two warps solve eight rows of the
+// strip's columns while the others apply the eight rows below to the rows above them.
+__device__ __forceinline__ void front_back(const double *d, int ldd, int m, double *b, int ldb, int nb, const double *rpiv,
                                            bool extreme)
 {
     const int tid = threadIdx.x, warp = tid >> 5, nw = kFrontThreads / 32;
+#pragma unroll 1
     for (int r0 = (m - 1) / kPanel * kPanel; r0 >= 0; r0 -= kPanel)
     {
-        const int w = min(kPanel, m - r0), r1 = r0 + kPanel;
+        const int w = min(kPanel, m - r0), r1 = r0 + kPanel, n = r0 / 8;
         if (warp < 2)
         {
-            double *col = b + r0 * kLdStrip + tid;
-            if (tid < 8 * nb && (extreme || !front_backward<false>(d + r0 * ldd + r0, ldd, rpiv + r0, col, kLdStrip, w)))
-                front_backward_divide(d + r0 * ldd + r0, ldd, col, kLdStrip, w);
+            double *col = b + r0 * ldb + tid;
+            if (tid < 8 * nb && (extreme || !front_backward<false>(d + r0 * ldd + r0, ldd, rpiv + r0, col, ldb, w)))
+                front_backward_divide(d + r0 * ldd + r0, ldd, col, ldb, w);
         }
         else if (r1 < m)
         {
-            for (int t = warp - 2; t < nb * ((r0 + 31) / 32); t += nw - 2)
+            for (int t = warp - 2; t < 2 * nb; t += nw - 2)
             {
-                const int c0 = 8 * (t % nb), row = t / nb * 32;
-                front_tiles<4, true>(b + c0, kLdStrip, d + r1, ldd, b + r1 * kLdStrip + c0, kLdStrip, row,
-                                     min(row + 32, r0), min(kPanel, m - r1));
+                const int c0 = 8 * (t >> 1);
+                front_tiles<true>(b + c0, ldb, d + r1, ldd, b + r1 * ldb + c0, ldb, t & 1 ? n >> 1 : 0, t & 1 ? n : n >> 1,
+                                  min(kPanel, m - r1));
             }
         }
         __syncthreads();
         if (r0 == 0)
             break;
         for (int t = warp; t < nb; t += nw)
-            front_tiles<1, true>(b + 8 * t, kLdStrip, d + r0, ldd, b + r0 * kLdStrip + 8 * t, kLdStrip, r0 - 8, r0, w);
+            front_tiles<true>(b + 8 * t, ldb, d + r0, ldd, b + r0 * ldb + 8 * t, ldb, n - 1, n, w);
         __syncthreads();
     }
 }
 
+// The update by the pivot before, of blocks in shared memory: d -= L Ud (nd tiles of eight columns, row stride
+// ldd; Ud: K x m, row-major) and b -= L Ub (nb tiles, row stride ldb; Ub: K x ldu, row-major, w columns of
+// it), L: rows x K in global memory, all at most 64 and rows at most 8 kTiles. Either may be absent (nd or
+// nb zero). A warp holds one column tile of d and its share of b's tiles in registers throughout;
+// `buf`: the operands of a step, loaded while the step before is computed. For 64 rows 13,400
+// cycles; with the tiles in shared memory 23,000, with the operands read straight from L1 and no
+// barriers 15,700.
+template <int kTiles, typename T>
+__device__ __forceinline__ void front_prev(double *d, int ldd, int m, int nd, double *b, int ldb, int nb, int w,
+                                           const T *__restrict__ L, int rows, const T *__restrict__ Ud,
+                                           const T *__restrict__ Ub, int ldu, int K, double *buf)
+{
+    constexpr int kPer = kPrevMax * kPrevK / kFrontThreads; // values of each operand per thread and step
+    constexpr int kLdD = front_ldb(kPrevMax);
+    double *sl = buf, *sd = sl + kPrevMax * kLdPrev, *sb = sd + kPrevK * kLdD;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
+    T rl[kPer], rd[kPer], rb[kPer];
+    auto load = [&](int k0) {
+#pragma unroll
+        for (int i = 0; i < kPer; ++i)
+        {
+            const int e = tid + i * kFrontThreads;
+            const int r = e / kPrevK, k = k0 + e % kPrevK;
+            rl[i] = r < rows && k < K ? L[r * K + k] : T(0);
+            const int kr = k0 + e / kPrevMax, c = e % kPrevMax;
+            rd[i] = nd > 0 && kr < K && c < m ? Ud[kr * m + c] : T(0);
+            rb[i] = nb > 0 && kr < K && c < w ? Ub[(int64_t)kr * ldu + c] : T(0);
+        }
+    };
+    load(0);
+    // the warp's tiles: column tile `warp` of d; of b column tile bc, row tiles bp, bp + share, ...
+    const int lb = nb == 1 ? 0 : nb == 2 ? 1 : nb <= 4 ? 2 : 3, share = 8 >> lb, bc = warp & ((1 << lb) - 1), bp = warp >> lb;
+    const bool has_d = warp < nd, has_b = bc < nb;
+    double *pd = d + g * ldd + 8 * warp + 2 * q, *pb = b + (8 * bp + g) * ldb + 8 * bc + 2 * q;
+    const int rt = (rows + 7) / 8;
+    double2 xd[kTiles], xb[kTiles];
+#pragma unroll
+    for (int i = 0; i < kTiles; ++i)
+    {
+        xd[i] = has_d && i < rt ? *reinterpret_cast<double2 *>(pd + 8 * i * ldd) : make_double2(0, 0);
+        xb[i] = has_b && bp + i * share < rt ? *reinterpret_cast<double2 *>(pb + 8 * i * share * ldb) : make_double2(0, 0);
+    }
+#pragma unroll 1
+    for (int k0 = 0; k0 < K; k0 += kPrevK)
+    {
+#pragma unroll
+        for (int i = 0; i < kPer; ++i)
+        {
+            const int e = tid + i * kFrontThreads;
+            sl[e / kPrevK * kLdPrev + e % kPrevK] = -(double)rl[i];
+            sd[e / kPrevMax * kLdD + e % kPrevMax] = (double)rd[i];
+            if (e % kPrevMax < ldb)
+                sb[e / kPrevMax * ldb + e % kPrevMax] = (double)rb[i];
+        }
+        __syncthreads();
+        if (k0 + kPrevK < K)
+            load(k0 + kPrevK);
+        // every tile's products, those beyond the rows on zeros: no test per tile
+        if (has_d)
+#pragma unroll
+            for (int s = 0; s < kPrevK / 4; ++s)
+            {
+                const double v = sd[(4 * s + q) * kLdD + 8 * warp + g];
+#pragma unroll
+                for (int i = 0; i < kTiles; ++i)
+                    dmma_8x8x4(xd[i].x, xd[i].y, sl[(8 * i + g) * kLdPrev + 4 * s + q], v);
+            }
+        if (has_b)
+        {
+            const double *a = sl + (8 * bp + g) * kLdPrev + q, *u = sb + q * ldb + 8 * bc + g;
+            if (share == 4)
+            {
+#pragma unroll
+                for (int s = 0; s < kPrevK / 4; ++s)
+#pragma unroll
+                    for (int i = 0; i < (kTiles + 3) / 4; ++i)
+                        dmma_8x8x4(xb[i].x, xb[i].y, a[32 * i * kLdPrev + 4 * s], u[4 * s * ldb]);
+            }
+            else
+            {
+                for (int s = 0; s < kPrevK / 4; ++s)
+#pragma unroll
+                    for (int i = 0; i < kTiles; ++i)
+                    {
+                        // tiles beyond the last of the eight repeat it; they are not stored
+                        const int row = min(i * share, 7 - bp);
+                        dmma_8x8x4(xb[i].x, xb[i].y, a[8 * row * kLdPrev + 4 * s], u[4 * s * ldb]);
+                    }
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < kTiles; ++i)
+    {
+        if (has_d && i < rt)
+            *reinterpret_cast<double2 *>(pd + 8 * i * ldd) = xd[i];
+        if (has_b && bp + i * share < rt)
+            *reinterpret_cast<double2 *>(pb + 8 * i * share * ldb) = xb[i];
+    }
+    __syncthreads();
+}
+
+// Index of v among the ascending a[b, e), -1 if it is not there; `guess` is looked at first.
+__device__ __forceinline__ int64_t front_find(const int32_t *a, int64_t b, int64_t e, int32_t v, int64_t guess)
+{
+    if (guess < e && a[guess] == v)
+        return guess;
+    const int64_t i = find_col(a, b, e, v);
+    return i < e && a[i] == v ? i : -1;
+}
+
+// BF16 splits (hyb_umma.cuh) of the 64-row strip b (row stride ldb): columns col0 .. col0 + w - 1 of an upper
+// block, transposed.
+__device__ __forceinline__ void front_split_upper(unsigned char *dst, const double *b, int ldb, int col0, int w)
+{
+    for (int e = threadIdx.x; e < 512; e += kFrontThreads)
+    {
+        const int c = e & 63, q = e >> 6;
+        if (c >= w)
+            continue;
+        float x[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            x[i] = (float)b[(q * 8 + i) * ldb + c];
+        uint4 hi, lo;
+        split8(x, hi, lo);
+        const uint32_t off = sw128_offset(col0 + c, q * 8);
+        *reinterpret_cast<uint4 *>(dst + off) = hi;
+        *reinterpret_cast<uint4 *>(dst + kSplitHalf + off) = lo;
+    }
+}
+
+// What the host knows of a level with one pivot (k >= 0) and of the pivot before it (kp >= 0, else none): indices
+// that the kernel would otherwise fetch one after the other.
+struct FrontOne
+{
+    int64_t k = -1, dpos = 0, end = 0, doff = 0; // pivot, filled index and offset of its diagonal block, end of its row
+    int64_t kp = -1, u0 = 0, uend = 0;           // pivot before, its upper blocks
+    int64_t l0 = 0, lend = 0;                    // its lower blocks (lcol_*)
+    int64_t loff = 0, udoff = 0;                 // offsets of the blocks (k, kp) and (kp, k)
+    int32_t m = 0, Kp = 0, ip = -1, jp = -1;     // sizes; k's place in kp's lower column and upper row, -1: absent
+};
+
+// The lower block of a column unit of k_front: row t of pivot k's column, the i-th from the top. With a pivot
+// before (o.kp) whose column holds row t, T(t,k) -= L(t,kp) U(kp,k); on a tensor-core level (ops) the
+// block's BF16 split and the slab offsets of row t's targets (as k_split64 leaves them).
+template <typename T>
+__device__ __forceinline__ void front_column(const DevSym &S, T *__restrict__ slab, int64_t p0, int64_t p, int64_t k,
+                                             int64_t i, const FrontOne &o, double *b, double *buf,
+                                             unsigned char *ops, int64_t *tgt)
+{
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = kFrontThreads / 32;
+    const int64_t e = S.lcol_ptr[k] + i;
+    const int32_t t = S.lcol_row[e];
+    T *g = slab + S.blk_off[S.lcol_blk[e]];
+    const int M = S.size[t], m = S.size[k], rows = front_rows(M), nb = (m + 7) / 8;
+    constexpr int ldb = front_ldb(kPrevMax);
+    int64_t el = -1;
+    if (o.kp >= 0 && o.jp >= 0)
+        el = front_find(S.lcol_row, o.l0, o.lend, t, o.l0 + max(o.ip + 1, 0) + i);
+    if (el < 0 && !ops)
+        return;
+    front_load(b, ldb, g, m, M, m, rows, 8 * nb, warp, nw);
+    __syncthreads();
+    if (el >= 0)
+    {
+        front_prev<8, T>(b, 0, 0, 0, b, ldb, nb, m, slab + S.blk_off[S.lcol_blk[el]], M, nullptr, slab + o.udoff, m,
+                         o.Kp, buf);
+        for (int r = warp; r < M; r += nw)
+            for (int c = lane; c < m; c += 32)
+                g[r * m + c] = (T)b[r * ldb + c];
+    }
+    if (!ops)
+        return;
+    unsigned char *dst = ops + (S.split_pref[p] - S.split_pref[p0] + i) * (int64_t)kSplitBytes;
+    for (int ch = tid; ch < 512; ch += kFrontThreads)
+    {
+        const int row = ch >> 3, q = ch & 7;
+        float x[8];
+#pragma unroll
+        for (int v = 0; v < 8; ++v)
+            x[v] = (float)b[row * ldb + q * 8 + v];
+        uint4 hi, lo;
+        split8(x, hi, lo);
+        const uint32_t off = sw128_offset(row, q * 8);
+        *reinterpret_cast<uint4 *>(dst + off) = hi;
+        *reinterpret_cast<uint4 *>(dst + kSplitHalf + off) = lo;
+    }
+    const int64_t n_up = S.row_ptr[k + 1] - S.diag_pos[k] - 1;
+    int64_t *row_tgt = tgt + (S.upd_pref[p] - S.upd_pref[p0]) + i * n_up;
+    for (int64_t j = tid; j < n_up; j += kFrontThreads)
+        row_tgt[j] = S.blk_off[find_col(S.cols, S.row_ptr[t], S.row_ptr[t + 1], S.cols[S.diag_pos[k] + 1 + j])];
+}
+
 // The level's pivots p0 .. p1 of up to 128 rows: grid.x the units of lu_pref (one per upper block
-// of a pivot, at least one per pivot), grid.y the strips (of 16, 32 or 64 columns) of the widest upper block. Each
-// CTA reads and factors its pivot's block; the one that takes the pivot's last ticket -- after
-// all have read it -- writes the factors back. The first CTA of a pivot reports zero and
+// of a pivot, at least one per pivot), grid.y the strips (of 16, 32 or 64 columns) of the widest upper
+// block. Each CTA reads and factors its pivot's block; the one that takes the pivot's last ticket
+// -- after all have read it -- writes the factors back. The first CTA of a pivot reports zero and
 // non-finite pivots and, with a growth limit (the mixed form), whether the pivot's growth
 // max|U| / max|D| passes it: counted as before by size, though the arithmetic is FP64 either way.
+//
+// With a pivot before (one.kp >= 0; single pivots of up to 64 rows, all blocks concerned at most 64 wide) its
+// update of the pivot's row and column is applied on the way: every CTA updates the
+// diagonal block it is about to factor and its strip, and n_lower column units beyond n_units take
+// the blocks below the diagonal. On a tensor-core level (ops) the column units are there for every
+// pivot and leave the update kernels' operands (BF16 splits, target table); the strips leave
+// their upper blocks' splits. A separate launch for the row and column took as long as the
+// factorization again, between two pivots of the chain.
 template <typename T>
 __global__ void __launch_bounds__(kFrontThreads, 2)
     k_front(DevSym S, T *__restrict__ slab, int64_t p0, int64_t p1, int *__restrict__ tickets, int *status,
-            float growth_limit, int strip)
+            float growth_limit, int strip, unsigned n_units, FrontOne one, unsigned char *ops, int64_t *tgt)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int s_writer, s_flags[2]; // a panel to be divided by its pivots; any such
-    const int tid = threadIdx.x;
-    const int64_t u = S.lu_pref[p0] + blockIdx.x;
-    const int64_t p = find_owner(S.lu_pref, p0, p1, u);
-    const int64_t first = S.lu_pref[p], k = S.piv[p];
-    const int64_t j = u - first, dpos = S.diag_pos[k], blk = dpos + 1 + j;
-    const int m = S.size[k], rows = front_rows(m), ldd = rows + 4;
-    const int cc = blk < S.row_ptr[k + 1] ? S.size[S.cols[blk]] : 0, col0 = strip * (int)blockIdx.y;
-    const int w = max(0, min(strip, cc - col0)), nb = (w + 7) / 8;
-    const int total = (int)(S.lu_pref[p + 1] - first) * (int)gridDim.y;
-    const bool owner = j == 0 && blockIdx.y == 0;
-    T *gd = slab + S.blk_off[dpos];
-    T *gb = slab + S.blk_off[blk] + col0; // read only where w > 0 (blk_off has one entry more than blocks)
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = kFrontThreads / 32;
     double *d = reinterpret_cast<double *>(smem_raw);
+    const bool prev = one.kp >= 0;
+    if (blockIdx.x >= n_units)
+    {
+        if (blockIdx.y > 0)
+            return;
+        // lower blocks of the level's pivots: n_lc = the split units less the upper blocks
+        const int64_t v = blockIdx.x - n_units, base = S.split_pref[p0] - S.trsm_pref[p0];
+        int64_t lo = p0, hi = p1;
+        while (hi - lo > 1)
+        {
+            const int64_t mid = (lo + hi) >> 1;
+            if (S.split_pref[mid] - S.trsm_pref[mid] - base <= v)
+                lo = mid;
+            else
+                hi = mid;
+        }
+        front_column<T>(S, slab, p0, lo, S.piv[lo], v - (S.split_pref[lo] - S.trsm_pref[lo] - base), one, d,
+                        d + kPrevMax * front_ldb(kPrevMax), ops, tgt);
+        return;
+    }
+    int64_t p = p0, k = one.k, j = blockIdx.x, dpos = one.dpos, end = one.end, doff = one.doff;
+    int m = one.m, total = (int)n_units * (int)gridDim.y;
+    if (k < 0)
+    {
+        const int64_t u = S.lu_pref[p0] + blockIdx.x;
+        p = find_owner(S.lu_pref, p0, p1, u);
+        j = u - S.lu_pref[p];
+        total = (int)(S.lu_pref[p + 1] - S.lu_pref[p]) * (int)gridDim.y;
+        k = S.piv[p];
+        m = S.size[k];
+        dpos = S.diag_pos[k];
+        end = S.row_ptr[k + 1];
+        doff = S.blk_off[dpos];
+    }
+    const int64_t blk = dpos + 1 + j;
+    const int rows = front_rows(m), ldd = rows + 4;
+    const int32_t c = blk < end ? S.cols[blk] : -1;
+    const int cc = c >= 0 ? S.size[c] : 0, col0 = strip * (int)blockIdx.y;
+    const int w = max(0, min(strip, cc - col0)), nb = (w + 7) / 8;
+    const bool owner = j == 0 && blockIdx.y == 0;
+    T *gd = slab + doff;
+    T *gb = slab + S.blk_off[blk] + col0; // read only where w > 0 (blk_off has one entry more than blocks)
     double *b = d + rows * ldd;
-    double *rpiv = b + rows * kLdStrip, *ubuf = rpiv + rows;
-    const int lane = tid & 31, warp = tid >> 5, nw = kFrontThreads / 32;
+    const int ldb = front_ldb(strip);
+    double *rpiv = b + rows * ldb, *ubuf = rpiv + rows, *uinv = ubuf + kPanel * kPanel;
 
     double amax = 0;
     for (int c0 = 0; c0 < rows; c0 += 64)
-        amax = fmax(amax, front_load(d + c0, ldd, gd + c0, m, m, m - c0, rows, min(64, rows - c0), warp, nw));
-    for (int i = m + tid; i < rows; i += kFrontThreads)
-        d[i * ldd + i] = 1;
+        amax = fmax(amax, front_load(d + c0, ldd, gd + c0, m, m, m - c0, rows, min(64, rows - c0), warp, nw, c0));
     if (tid < 2)
         s_flags[tid] = 0;
+    if (prev && nb > 0)
+        front_load(b, ldb, gb, cc, m, w, rows, 8 * nb, warp, nw);
     __syncthreads();
     if (tid == 0)
         s_writer = atomicAdd(tickets + p, 1) == total - 1;
-    const bool check = owner && std::is_same_v<T, float> && growth_limit > 0;
-    if (check)
-        amax = cta_max(amax);
     if (w == 0 && !owner)
     {
         // a strip beyond this block's width: the factors may still be this CTA's to write
@@ -463,20 +795,56 @@ __global__ void __launch_bounds__(kFrontThreads, 2)
         if (!s_writer)
             return;
     }
-    front_factor(d, ldd, m, b, nb, rpiv, ubuf, s_flags,
-                 [&](int wi, int n) { front_load(b, kLdStrip, gb, cc, m, w, rows, 8 * nb, wi, n); });
+    if (prev && one.ip >= 0)
+    {
+        const int64_t uc = nb > 0 ? front_find(S.cols, one.u0, one.uend, c, one.u0 + one.jp + 1 + j) : -1;
+        if (one.jp >= 0 || uc >= 0)
+        {
+            const int nd = one.jp >= 0 ? (m + 7) / 8 : 0, nu = uc >= 0 ? nb : 0;
+            const T *ub = slab + (uc >= 0 ? S.blk_off[uc] + col0 : 0);
+            double *buf = uinv + rows * kLdUinv;
+            if (m <= 32)
+                front_prev<4, T>(d, ldd, m, nd, b, ldb, nu, w, slab + one.loff, m, slab + one.udoff, ub, cc, one.Kp, buf);
+            else
+                front_prev<8, T>(d, ldd, m, nd, b, ldb, nu, w, slab + one.loff, m, slab + one.udoff, ub, cc, one.Kp, buf);
+        }
+    }
+    const bool check = owner && std::is_same_v<T, float> && growth_limit > 0;
+    if (check)
+    {
+        if (prev) // the block that is factored
+        {
+            amax = 0;
+            for (int i = tid; i < m * m; i += kFrontThreads)
+                amax = fmax(amax, fabs(d[i / m * ldd + i % m]));
+        }
+        amax = cta_max(amax);
+    }
+    const bool exact = m <= kExactMax;
+    front_factor(d, ldd, m, b, ldb, nb, rpiv, ubuf, s_flags, exact ? nullptr : uinv, [&](int wi, int n) {
+        if (!prev)
+            front_load(b, ldb, gb, cc, m, w, rows, 8 * nb, wi, n);
+    });
     if (nb > 0)
     {
-        front_back(d, ldd, m, b, nb, rpiv, s_flags[1] != 0);
+        // extreme pivots and values that are not finite: by divisions
+        if (exact || s_flags[1] != 0)
+            front_back(d, ldd, m, b, ldb, nb, rpiv, s_flags[1] != 0);
+        else
+            front_back_products(d, ldd, m, b, ldb, nb, uinv);
         for (int r = warp; r < m; r += nw)
-            for (int c = lane; c < w; c += 32)
-                gb[(int64_t)r * cc + c] = (T)b[r * kLdStrip + c];
+            for (int q = lane; q < w; q += 32)
+                gb[(int64_t)r * cc + q] = (T)b[r * ldb + q];
+        if (ops)
+            front_split_upper(ops + (S.split_pref[p] - S.split_pref[p0] + S.lcol_ptr[k + 1] - S.lcol_ptr[k] + j) *
+                                        (int64_t)kSplitBytes,
+                              b, ldb, col0, w);
     }
     if (s_writer)
     {
         for (int r = warp; r < m; r += nw)
-            for (int c = lane; c < m; c += 32)
-                gd[r * m + c] = (T)d[r * ldd + c];
+            for (int q = lane; q < m; q += 32)
+                gd[r * m + q] = (T)d[r * ldd + q];
         if (tid == 0)
             tickets[p] = 0; // ready for the next factorization
     }

@@ -524,7 +524,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1)
         FlowDiag<T> dg;
         for (int ch = 0; ch < nrhs; ch += NC)
         {
-            const int nc = min(NC, nrhs - ch);
+            const int nc = NC == 1 ? 1 : min(NC, nrhs - ch);
             for (int r0 = 0; r0 < m; r0 += rows)
             {
                 FlowBlock<T> cur, nxt;
@@ -692,7 +692,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1)
     const int tpr = gemv_tpr<T>(m), rows = kFlowThreads / tpr, q = tid & (tpr - 1);
     for (int ch = 0; ch < nrhs; ch += NC)
     {
-        const int nc = min(NC, nrhs - ch);
+        const int nc = NC == 1 ? 1 : min(NC, nrhs - ch);
         for (int r0 = 0; r0 < m; r0 += rows)
         {
             FlowSum<T, NC> a = {};
@@ -728,7 +728,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1)
         flow_diag_load(dg, S, slab, wbuf, f.k, m, tpr, sm.d, stage);
     for (int ch = 0; ch < nrhs; ch += NC)
     {
-        const int nc = min(NC, nrhs - ch);
+        const int nc = NC == 1 ? 1 : min(NC, nrhs - ch);
         for (int e = tid; e < m * nc; e += kFlowThreads)
         {
             const int64_t at = (int64_t)(e / nc) * nrhs + ch + e % nc;
@@ -762,6 +762,8 @@ __global__ void __launch_bounds__(kFlowThreads, 1)
 // X = D_k^{-1} and W(k,s) = D_k^{-1} L(k,s) for the late blocks of the pivots that keep them, in FP64, once
 // the factors are final. grid.x: the blocks (w_blk < 0: X), grid.y: their 64-column strips. Throughput only (one launch, off
 // the chain): 0.1 ms per 1,000 blocks of 64x64 on a B200.
+constexpr int kLdLate = front_ldb(64);
+
 template <typename T>
 __global__ void __launch_bounds__(kFrontThreads, 2) k_late(DevSym S, const T *__restrict__ slab, T *__restrict__ wbuf)
 {
@@ -773,7 +775,7 @@ __global__ void __launch_bounds__(kFrontThreads, 2) k_late(DevSym S, const T *__
     if (col0 >= K || !flow_uses_w<T>(m))
         return;
     const int w = min(64, K - col0), nb = (w + 7) / 8, rows = front_rows(m), ldd = rows + 4;
-    double *d = reinterpret_cast<double *>(smem_raw), *b = d + rows * ldd, *rpiv = b + rows * kLdStrip;
+    double *d = reinterpret_cast<double *>(smem_raw), *b = d + rows * ldd, *rpiv = b + rows * kLdLate;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = kFrontThreads / 32;
     const T *gd = slab + S.blk_off[S.diag_pos[k]];
     if (tid == 0)
@@ -781,11 +783,11 @@ __global__ void __launch_bounds__(kFrontThreads, 2) k_late(DevSym S, const T *__
     for (int c0 = 0; c0 < rows; c0 += 64)
         front_load(d + c0, ldd, gd + c0, m, m, m - c0, rows, min(64, rows - c0), warp, nw);
     if (blk >= 0)
-        front_load(b, kLdStrip, slab + S.blk_off[blk] + col0, K, m, w, rows, 8 * nb, warp, nw);
+        front_load(b, kLdLate, slab + S.blk_off[blk] + col0, K, m, w, rows, 8 * nb, warp, nw);
     else
         for (int r = warp; r < rows; r += nw)
             for (int c = lane; c < 8 * nb; c += 32)
-                b[r * kLdStrip + c] = r == col0 + c;
+                b[r * kLdLate + c] = r == col0 + c;
     __syncthreads();
     if (tid < m)
     {
@@ -798,21 +800,22 @@ __global__ void __launch_bounds__(kFrontThreads, 2) k_late(DevSym S, const T *__
     for (int r0 = 0; r0 < m; r0 += kPanel)
     {
         if (tid < 8 * nb)
-            front_forward(d + r0 * ldd + r0, ldd, b + r0 * kLdStrip + tid, kLdStrip);
+            front_forward(d + r0 * ldd + r0, ldd, b + r0 * kLdLate + tid, kLdLate);
         __syncthreads();
-        const int r1 = r0 + kPanel;
-        for (int t = warp; t < nb * ((rows - r1 + 31) / 32); t += nw)
+        const int r1 = r0 + kPanel, n = (rows - r1) / 8;
+        for (int t = warp; t < 2 * nb; t += nw)
         {
-            const int c0 = 8 * (t % nb), row = r1 + t / nb * 32;
-            front_tiles<4>(b + c0, kLdStrip, d + r0, ldd, b + r0 * kLdStrip + c0, kLdStrip, row, min(row + 32, rows));
+            const int c0 = 8 * (t >> 1);
+            front_tiles(b + r1 * kLdLate + c0, kLdLate, d + r1 * ldd + r0, ldd, b + r0 * kLdLate + c0, kLdLate,
+                        t & 1 ? n >> 1 : 0, t & 1 ? n : n >> 1);
         }
         __syncthreads();
     }
-    front_back(d, ldd, m, b, nb, rpiv, s_extreme != 0);
+    front_back(d, ldd, m, b, kLdLate, nb, rpiv, s_extreme != 0);
     T *out = wbuf + S.w_out[blockIdx.x] + col0;
     for (int r = warp; r < m; r += nw)
         for (int c = lane; c < w; c += 32)
-            out[(int64_t)r * K + c] = (T)b[r * kLdStrip + c];
+            out[(int64_t)r * K + c] = (T)b[r * kLdLate + c];
 }
 
 } // namespace hyb

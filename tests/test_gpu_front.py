@@ -99,3 +99,46 @@ def test_overflowing_quotient_stays_infinite(gpu):
     ns = gpu.NativeSystem.from_matrix(mat)
     ns.decompose(gpu.FP64)
     assert ns.get_block(0, 0, (2, 2))[1, 0] == np.inf
+
+
+# blocks of at most 64 rows: each pivot's kernel applies the pivot before to its own row and column
+# (contraction in steps of 16, tiles of 8, strips of 16 and 32 columns)
+@pytest.mark.parametrize("m", [1, 7, 8, 9, 15, 16, 17, 33, 48, 63, 64])
+def test_update_by_the_pivot_before_matches_oracle(gpu, m):
+    mat = _dense_blocks([m, 1, m, 64, 33, 8, m, 20], seed=100 + m)
+    osys = O.OracleSystem.from_csr(mat.sizes, mat.row_ptr, mat.cols, mat.vals)
+    osys.decompose()
+    ns = gpu.NativeSystem.from_matrix(mat)
+    ns.decompose(gpu.FP64)
+    first = _factors(ns, mat)
+    for i, row in enumerate(first):
+        for c, got in enumerate(row):
+            assert rel_err(got, osys.get_block(i, c)) < 1e-12, (i, c)
+    for _ in range(3):  # no value depends on which warp or CTA is first
+        ns.set_values(mat.vals)
+        ns.decompose(gpu.FP64)
+        for row, ref in zip(_factors(ns, mat), first):
+            for got, want in zip(row, ref):
+                assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("n", [2, 3, 6, 46])
+def test_tensor_core_pivots_on_both_sides_of_the_rule(gpu, n):
+    """64-row pivots of the mixed form with few upper blocks (k_front, its pairs) and with many: every
+    stored FP32 value is rounded once per pivot that updates it, and the split products keep 2^-16
+    or better, n of them."""
+    mat = _dense_blocks([64] * n, seed=n)
+    ns = gpu.NativeSystem.from_matrix(mat)
+    ns.set_option(gpu.OPTION_BLOCK_SCALING, 0)
+    ns.decompose(gpu.FP64)
+    f64 = _factors(ns, mat)
+    info = ns.decompose(gpu.MIXED)
+    assert info["zero_pivots"] == 0 and info["non_finite"] == 0
+    first = _factors(ns, mat)
+    for row, ref in zip(first, f64):
+        for got, want in zip(row, ref):
+            assert rel_err(got, want) < 1e-4
+    ns.decompose(gpu.MIXED)
+    for row, ref in zip(_factors(ns, mat), first):
+        for got, want in zip(row, ref):
+            assert np.array_equal(got, want)
