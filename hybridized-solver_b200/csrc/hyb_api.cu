@@ -137,7 +137,7 @@ enum UpdateKernel
 {
     UPD_TILE32 = 0, // k_update32: 64-thread CTAs of one 32x32 output tile (targets up to 256 wide)
     UPD_TILE64 = 1, // k_update: one 256-thread CTA per target, its 64x64 tiles in turn
-    UPD_DMMA = 2,   // k_update_dmma: FP64 tensor pipe, one CTA per 64x64 tile (pivots up to 128 rows)
+    UPD_DMMA = 2,   // k_update_dmma: FP64 tensor pipe, 64-column strips (pivots up to 128 rows)
     UPD_KINDS = 3
 };
 
@@ -844,8 +844,8 @@ int level_bucket(const Symbolic::LevelShape &sh)
 }
 
 // The generic update kernel of level l: the forced one (HYB_OPTION_UPDATE_KERNEL) where it
-// fits, else the tuned choice of the level's size bucket, else the fixed rule (32x32 tiles
-// for targets up to 256 wide, 64x64 tiles beyond).
+// fits, else the tuned choice of the level's size bucket, else the fixed rule (the FP64 tensor
+// pipe for pivots it takes, then 32x32 tiles for targets up to 256 wide, 64x64 tiles beyond).
 template <typename T> int generic_kernel(const hyb_system *h, int64_t l)
 {
     const Symbolic::LevelShape &sh = h->S.shape[l];
@@ -854,7 +854,7 @@ template <typename T> int generic_kernel(const hyb_system *h, int64_t l)
     const int tuned = h->tuned[std::is_same_v<T, float> ? 1 : 0][level_bucket(sh)];
     if (tuned >= 0 && generic_kernel_fits(sh, tuned))
         return tuned;
-    return generic_kernel_fits(sh, UPD_TILE32) ? UPD_TILE32 : UPD_TILE64;
+    return generic_kernel_fits(sh, UPD_DMMA) ? UPD_DMMA : generic_kernel_fits(sh, UPD_TILE32) ? UPD_TILE32 : UPD_TILE64;
 }
 
 template <typename T>
@@ -878,9 +878,28 @@ int enqueue_generic_update(hyb_system *h, T *slab, int64_t l, cudaStream_t st, i
     }
     if (kind == UPD_DMMA)
     {
-        const unsigned t64 = (unsigned)(((sh.max_row + 63) / 64) * ((sh.max_col + 63) / 64));
-        hyb::k_update_dmma<T><<<dim3((unsigned)nu, t64), hyb::kDmmaThreads, hyb::dmma_smem_bytes(sh.max_piv), st>>>(
-            ds, slab, p0, p1, mode, sh.la_i0, sh.la_j0);
+        // the upper blocks' strips, their rows shared out so that each CTA has about two 16-row slices per
+        // warp; one where that leaves SMs with less than they can hold
+        const int64_t upper = S.trsm_pref[p1] - S.trsm_pref[p0], strips = (sh.max_col + hyb::kDmmaStrip - 1) / hyb::kDmmaStrip;
+        const int64_t lower = (S.split_pref[p1] - S.split_pref[p0] - upper + p1 - p0 - 1) / (p1 - p0);
+        const int64_t slices = lower * ((sh.max_row + 15) / 16);
+        constexpr int64_t kWarps = hyb::kDmmaThreads / 32;
+        int64_t cols = upper, shares = (slices + 2 * kWarps - 1) / (2 * kWarps);
+        if (upper * strips * shares < hyb::kDmmaCtas * sm_count())
+            shares = (slices + kWarps - 1) / kWarps;
+        shares = std::max<int64_t>(1, std::min(shares, lower));
+        if (mode == 1)
+        {
+            shares = lower;
+            cols = (sh.la_i0 >= 0 ? upper : 0) + (sh.la_j0 >= 0 ? shares : 0);
+        }
+        else if (mode == 2 && sh.la_j0 >= 0)
+        {
+            --cols;
+        }
+        hyb::k_update_dmma<T><<<dim3((unsigned)cols, (unsigned)strips, mode == 1 ? 1 : (unsigned)shares), hyb::kDmmaThreads,
+                                hyb::dmma_smem_bytes(sh.max_piv), st>>>(ds, slab, p0, p1, mode, sh.la_i0, sh.la_j0,
+                                                                        (int)shares);
         ++launches;
         HYB_LAUNCHED("k_update_dmma", l);
         return HYB_SUCCESS;
@@ -1180,9 +1199,11 @@ template <typename T> int enqueue_factor(hyb_system *h, T *slab, uint64_t &launc
         };
         if (lookahead)
         {
-            // FP64: the next pivot's kernel updates its row and column itself. (FP32 updates are rounded by
-            // the kernel that makes them, and lookahead does not change the factors.)
-            const bool taken = std::is_same_v<T, double> && !pair && front_takes<T>(h, l, next);
+            // The next pivot's kernel updates its row and column itself, in FP64: not where the rest of an FP32
+            // update is summed in FP32 or on the tensor cores, as lookahead does not change the factors.
+            const bool taken = !pair && front_takes<T>(h, l, next) &&
+                               (std::is_same_v<T, double> ||
+                                (!tc_level<T>(h, l) && generic_kernel<T>(h, l) == UPD_DMMA));
             if (!taken && (rc = update(1)) != HYB_SUCCESS)
                 return rc;
             HYB_CUDA(cudaEventRecord(h->ev_prio, st));

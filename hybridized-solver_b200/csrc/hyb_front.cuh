@@ -518,7 +518,8 @@ __device__ __forceinline__ void front_back(const double *d, int ldd, int m, doub
 // ldd; Ud: K x m, row-major) and b -= L Ub (nb tiles, row stride ldb; Ub: K x ldu, row-major, w columns of
 // it), L: rows x K in global memory, all at most 64 and rows at most 8 kTiles. Either may be absent (nd or
 // nb zero). A warp holds one column tile of d and its share of b's tiles in registers throughout;
-// `buf`: the operands of a step, loaded while the step before is computed. For 64 rows 13,400
+// `buf`: the operands of a step, loaded while the step before is computed. The sums are FP64 and rounded to T
+// once, as by the generic update kernel. For 64 rows 13,400
 // cycles; with the tiles in shared memory 23,000, with the operands read straight from L1 and no
 // barriers 15,700.
 template <int kTiles, typename T>
@@ -610,20 +611,11 @@ __device__ __forceinline__ void front_prev(double *d, int ldd, int m, int nd, do
     for (int i = 0; i < kTiles; ++i)
     {
         if (has_d && i < rt)
-            *reinterpret_cast<double2 *>(pd + 8 * i * ldd) = xd[i];
+            *reinterpret_cast<double2 *>(pd + 8 * i * ldd) = make_double2((T)xd[i].x, (T)xd[i].y);
         if (has_b && bp + i * share < rt)
-            *reinterpret_cast<double2 *>(pb + 8 * i * share * ldb) = xb[i];
+            *reinterpret_cast<double2 *>(pb + 8 * i * share * ldb) = make_double2((T)xb[i].x, (T)xb[i].y);
     }
     __syncthreads();
-}
-
-// Index of v among the ascending a[b, e), -1 if it is not there; `guess` is looked at first.
-__device__ __forceinline__ int64_t front_find(const int32_t *a, int64_t b, int64_t e, int32_t v, int64_t guess)
-{
-    if (guess < e && a[guess] == v)
-        return guess;
-    const int64_t i = find_col(a, b, e, v);
-    return i < e && a[i] == v ? i : -1;
 }
 
 // BF16 splits (hyb_umma.cuh) of the 64-row strip b (row stride ldb): columns col0 .. col0 + w - 1 of an upper
@@ -674,7 +666,7 @@ __device__ __forceinline__ void front_column(const DevSym &S, T *__restrict__ sl
     constexpr int ldb = front_ldb(kPrevMax);
     int64_t el = -1;
     if (o.kp >= 0 && o.jp >= 0)
-        el = front_find(S.lcol_row, o.l0, o.lend, t, o.l0 + max(o.ip + 1, 0) + i);
+        el = find_near(S.lcol_row, o.l0, o.lend, t, o.l0 + max(o.ip + 1, 0) + i);
     if (el < 0 && !ops)
         return;
     front_load(b, ldb, g, m, M, m, rows, 8 * nb, warp, nw);
@@ -797,7 +789,7 @@ __global__ void __launch_bounds__(kFrontThreads, 2)
     }
     if (prev && one.ip >= 0)
     {
-        const int64_t uc = nb > 0 ? front_find(S.cols, one.u0, one.uend, c, one.u0 + one.jp + 1 + j) : -1;
+        const int64_t uc = nb > 0 ? find_near(S.cols, one.u0, one.uend, c, one.u0 + one.jp + 1 + j) : -1;
         if (one.jp >= 0 || uc >= 0)
         {
             const int nd = one.jp >= 0 ? (m + 7) / 8 : 0, nu = uc >= 0 ? nb : 0;

@@ -96,6 +96,20 @@ __device__ __forceinline__ int64_t find_owner(const int64_t *pref, int64_t lo, i
     return lo;
 }
 
+// The same by a whole warp, 32 ways at a time (all lanes call it with the same arguments; pref[lo] <= u).
+__device__ __forceinline__ int64_t warp_find_owner(const int64_t *pref, int64_t lo, int64_t hi, int64_t u)
+{
+    const int lane = threadIdx.x & 31;
+    while (hi - lo > 1)
+    {
+        const int64_t step = (hi - lo + 31) >> 5, at = lo + lane * step;
+        const int n = __popc(__ballot_sync(0xffffffffu, at < hi && pref[at] <= u));
+        lo += (n - 1) * step;
+        hi = min(hi, lo + step);
+    }
+    return lo;
+}
+
 // Index of column c in the sorted range cols[b, e) (the caller guarantees presence).
 __device__ __forceinline__ int64_t find_col(const int32_t *cols, int64_t b, int64_t e, int32_t c)
 {
@@ -110,7 +124,16 @@ __device__ __forceinline__ int64_t find_col(const int32_t *cols, int64_t b, int6
     return b;
 }
 
-// The same search by a whole warp (all lanes call it with the same arguments): each round
+// Index of v among the ascending a[b, e), -1 if it is not there; `guess` is looked at first.
+__device__ __forceinline__ int64_t find_near(const int32_t *a, int64_t b, int64_t e, int32_t v, int64_t guess)
+{
+    if (guess < e && a[guess] == v)
+        return guess;
+    const int64_t i = find_col(a, b, e, v);
+    return i < e && a[i] == v ? i : -1;
+}
+
+// The search of find_col by a whole warp (all lanes call it with the same arguments): each round
 // reads 256 entries with independent loads and finds c by ballot, so a row of up to 256
 // blocks costs one memory round trip instead of a chain of dependent ones.
 __device__ __forceinline__ int64_t warp_find_col(const int32_t *cols, int64_t b, int64_t e, int32_t c)
@@ -1431,100 +1454,219 @@ __global__ void __launch_bounds__(kUpd64Threads)
                 make_double2(acc[mi][ni][0], acc[mi][ni][1]);
 }
 
-// Generic-size Schur update on the FP64 tensor pipe (DMMA m8n8k4), for levels whose blocks
-// are not all 64 wide (uneven orders): one CTA per 64x64 tile of a target block (grid.y:
-// the tiles of the level's largest target; CTAs past a target's last tile return),
-// C(t,c)[tile] -= A(t,k) B(k,c) with A m x K and B K x n of any size, K <= kDmmaMaxK. The
-// operands are staged in shared memory as FP64, zero-padded to 64 rows/columns and to K
-// rounded up to 4 (padding adds exact zeros), C is held in DMMA accumulator fragments with
-// masked loads and stores; eight warps of 16x32 as in k_update64_f64. With T = float (the
-// mixed form's FP32 factors) the products are still formed in FP64 and rounded once.
+// Generic-size Schur update on the FP64 tensor pipe (DMMA m8n8k4), for blocks of any size and pivots of up
+// to kDmmaMaxK rows: C(t,c) -= A(t,k) U(k,c). A CTA keeps one strip of up to 32 columns of U(k,c) in shared
+// memory (as FP64, zero-padded) and takes a share of the rows t of the pivot's lower column: each warp, on
+// its own, 16 rows of a target at a time, its part of A straight from global memory as the products'
+// left operands and the target in accumulators; there is no barrier per target. With T = float the
+// products are formed in FP64 and rounded once.
+// It is bound by latency: a CTA's seven or so dependent loads for its indices, then a slice's loads of A and
+// of the target (long-scoreboard stalls half of the time, FP64 tensor pipe 20% busy). So: small CTAs, five
+// to an SM and each with about two slices per warp, rather than few that keep their strip longer; and
+// 32 columns, since 102 registers hold no more accumulators. Factorizations with one CTA per 64x64 tile of
+// a target or 32x32 tiles on the CUDA cores, and with this kernel: 25x25 p=6 13.3 and 12.3 ms, 32x32 of
+// orders 2..10 53.8 and 42.9 ms (half of it the row and column on the way to the next pivot, 24 us per
+// level with 32x32 tiles), 24 mixed systems of up to 24x24 41.0 and 30.9 ms. With 40 columns 12.9, 50.7 and 34.7 ms,
+// with 256 threads three to an SM 12.4, 45.6 and 30.8 ms.
 constexpr int kDmmaMaxK = 128;
-constexpr int kDmmaThreads = 256;
-
-__host__ __device__ constexpr int dmma_lda(int kp)
-{
-    return (kp + 15) / 16 * 16 + 4; // 64 + 4 for K = 64: the conflict-free stride of k_update64_f64
-}
+constexpr int kDmmaThreads = 128;
+constexpr int kDmmaCtas = 5; // per SM
+constexpr int kDmmaStrip = 32;
+constexpr int kDmmaLd = kDmmaStrip + 4; // conflict-free right operands
+constexpr int kDmmaBlocks = 64;         // lower blocks whose places are looked up at once
 
 __host__ __device__ constexpr int dmma_smem_bytes(int k)
 {
-    return (64 * dmma_lda((k + 3) / 4 * 4) + (k + 3) / 4 * 4 * kLd64) * 8;
+    return (k + 7) / 8 * 8 * kDmmaLd * 8;
 }
 
+// Values at p[0], p[1] of a row with `left` columns from p on; `pair`: p is aligned to two.
+template <typename T> __device__ __forceinline__ double2 dmma_load2(const T *p, int left, bool pair)
+{
+    if (pair && left >= 2)
+    {
+        using V = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
+        const V v = *reinterpret_cast<const V *>(p);
+        return make_double2((double)v.x, (double)v.y);
+    }
+    return make_double2(left > 0 ? (double)p[0] : 0.0, left > 1 ? (double)p[1] : 0.0);
+}
+
+template <typename T> __device__ __forceinline__ void dmma_store2(T *p, double2 v, int left, bool pair)
+{
+    if (pair && left >= 2)
+    {
+        if constexpr (sizeof(T) == 8)
+            *reinterpret_cast<double2 *>(p) = v;
+        else
+            *reinterpret_cast<float2 *>(p) = make_float2((float)v.x, (float)v.y);
+        return;
+    }
+    if (left > 0)
+        p[0] = (T)v.x;
+    if (left > 1)
+        p[1] = (T)v.y;
+}
+
+// Rows row0 .. row0 + 15 of one target's strip (n columns in kTiles column tiles) by one warp: A is M x K,
+// the target's row stride N.
+template <int kTiles, typename T>
+__device__ __forceinline__ void dmma_slice(const T *__restrict__ ga, T *__restrict__ gc, int row0, int M, int N, int n, int K,
+                                           const double *sb)
+{
+    const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+    const int r0 = row0 + g, r1 = r0 + 8;
+    const bool on0 = r0 < M, on1 = r1 < M, pair = (N & 1) == 0;
+    const T *pa = ga + r0 * K + q;
+    T a0[4], a1[4];
+    auto load = [&](int k0) {
+#pragma unroll
+        for (int s = 0; s < 4; ++s)
+        {
+            const int k = k0 + 4 * s;
+            a0[s] = on0 && k + q < K ? pa[k] : T(0);
+            a1[s] = on1 && k + q < K ? pa[8 * K + k] : T(0);
+        }
+    };
+    load(0);
+    T *c0 = gc + r0 * N + 2 * q, *c1 = c0 + 8 * N;
+    double2 v0[kTiles], v1[kTiles];
+#pragma unroll
+    for (int t = 0; t < kTiles; ++t)
+    {
+        v0[t] = dmma_load2(c0 + 8 * t, on0 ? n - 8 * t - 2 * q : 0, pair);
+        v1[t] = dmma_load2(c1 + 8 * t, on1 ? n - 8 * t - 2 * q : 0, pair);
+    }
+#pragma unroll 1
+    for (int k0 = 0; k0 < K; k0 += 16)
+    {
+        double x0[4], x1[4];
+#pragma unroll
+        for (int s = 0; s < 4; ++s)
+        {
+            x0[s] = -(double)a0[s];
+            x1[s] = -(double)a1[s];
+        }
+        if (k0 + 16 < K)
+            load(k0 + 16);
+        const double *pb = sb + (k0 + q) * kDmmaLd + g;
+#pragma unroll
+        for (int s = 0; s < 4; ++s)
+        {
+            if (s == 2 && k0 + 8 >= K) // uniform
+                break;
+#pragma unroll
+            for (int t = 0; t < kTiles; ++t)
+            {
+                const double u = pb[4 * s * kDmmaLd + 8 * t];
+                dmma_8x8x4(v0[t].x, v0[t].y, x0[s], u);
+                dmma_8x8x4(v1[t].x, v1[t].y, x1[s], u);
+            }
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < kTiles; ++t)
+    {
+        dmma_store2(c0 + 8 * t, v0[t], on0 ? n - 8 * t - 2 * q : 0, pair);
+        dmma_store2(c1 + 8 * t, v1[t], on1 ? n - 8 * t - 2 * q : 0, pair);
+    }
+}
+
+// grid.x: the upper blocks of the level's pivots, grid.y: their strips, grid.z: the shares of the
+// lower blocks. Of a single pivot, in mode 2 without the upper block j0 and the lower block i0, in mode 1
+// those alone: grid.x units of row i0 (if any), then `shares` units of column j0 (if any).
 template <typename T>
-__global__ void __launch_bounds__(kDmmaThreads)
-    k_update_dmma(DevSym S, T *__restrict__ slab, int64_t p0, int64_t p1, int mode, int i0, int j0)
+__global__ void __launch_bounds__(kDmmaThreads, kDmmaCtas)
+    k_update_dmma(DevSym S, T *__restrict__ slab, int64_t p0, int64_t p1, int mode, int i0, int j0, int shares)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const UpdUnit w = update_unit(S, p0, p1, mode, i0, j0, blockIdx.x);
-    const int32_t t = S.lcol_row[w.li];
-    const int32_t c = S.cols[w.bu];
-    const int M = S.size[t], N = S.size[c], K = S.size[w.k];
-    const int tn = (N + 63) / 64, tm = (M + 63) / 64;
-    if ((int)blockIdx.y >= tm * tn)
+    __shared__ int s_m[kDmmaBlocks];
+    __shared__ int64_t s_a[kDmmaBlocks], s_c[kDmmaBlocks];
+    double *sb = reinterpret_cast<double *>(smem_raw);
+    int64_t p = p0, j = blockIdx.x;
+    if (mode == 0)
+    {
+        const int64_t u = S.trsm_pref[p0] + blockIdx.x;
+        p = warp_find_owner(S.trsm_pref, p0, p1, u);
+        j = u - S.trsm_pref[p];
+    }
+    const int64_t k = S.piv[p], b0 = S.diag_pos[k] + 1, e0 = S.lcol_ptr[k];
+    const int n_lc = (int)(S.lcol_ptr[k + 1] - e0);
+    // the lower blocks first, first + step, ... of n_lc without `skip`
+    int first = blockIdx.z, step = shares, skip = -1, last = n_lc;
+    if (mode == 1)
+    {
+        const int64_t n_up = i0 >= 0 ? S.row_ptr[k + 1] - b0 : 0;
+        if (j < n_up)
+        {
+            first = i0;
+            last = i0 + 1;
+        }
+        else
+        {
+            first = (int)(j - n_up);
+            skip = i0;
+            j = j0;
+        }
+    }
+    else if (mode == 2)
+    {
+        j += j0 >= 0 && j >= j0;
+        skip = i0;
+    }
+    last -= skip >= 0;
+    const int64_t bu = b0 + j;
+    const int32_t c = S.cols[bu];
+    const int K = S.size[k], N = S.size[c], ns_c = (N + kDmmaStrip - 1) / kDmmaStrip;
+    const int width = ((N + ns_c - 1) / ns_c + 7) / 8 * 8, col0 = width * (int)blockIdx.y; // strips of much the same width
+    if (col0 >= N)
         return;
-    const int r0 = (blockIdx.y / tn) * 64, c0 = (blockIdx.y % tn) * 64;
-    const int mt = min(64, M - r0), nt = min(64, N - c0);
-    const int Kp = (K + 3) & ~3, lda = dmma_lda(Kp);
-    double *sa = reinterpret_cast<double *>(smem_raw); // 64 x lda: A rows r0.., K columns
-    double *sb = sa + 64 * lda;                        // Kp x kLd64: B rows, columns c0..
-    const int64_t tgt = warp_find_col(S.cols, S.row_ptr[t], S.row_ptr[t + 1], c);
-    const T *ga = slab + S.blk_off[S.lcol_blk[w.li]] + (int64_t)r0 * K;
-    const T *gb = slab + S.blk_off[w.bu] + c0;
-    T *gc = slab + S.blk_off[tgt] + (int64_t)r0 * N + c0;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int i = tid; i < 64 * Kp; i += kDmmaThreads)
-    {
-        const int r = i / Kp, q = i - r * Kp;
-        sa[r * lda + q] = (r < mt && q < K) ? -(double)ga[(int64_t)r * K + q] : 0.0;
-    }
-    for (int i = tid; i < Kp * 64; i += kDmmaThreads)
-    {
-        const int q = i >> 6, cc = i & 63;
-        sb[q * kLd64 + cc] = (q < K && cc < nt) ? (double)gb[(int64_t)q * N + cc] : 0.0;
-    }
-    const int g = lane >> 2, qq = lane & 3;
-    const int wm = (warp >> 1) * 16, wn = (warp & 1) * 32;
-    double acc[2][4][2];
-#pragma unroll
-    for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-            for (int e = 0; e < 2; ++e)
-            {
-                const int r = wm + mi * 8 + g, cc = wn + ni * 8 + 2 * qq + e;
-                acc[mi][ni][e] = (r < mt && cc < nt) ? (double)gc[(int64_t)r * N + cc] : 0.0;
-            }
-    __syncthreads();
+    const int n = min(width, N - col0), nt = (n + 7) / 8, Kp = (K + 7) / 8 * 8;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const T *gu = slab + S.blk_off[bu] + col0;
 #pragma unroll 4
-    for (int kk = 0; kk < Kp; kk += 4)
+    for (int r = warp; r < Kp; r += kDmmaThreads / 32)
+        sb[r * kDmmaLd + lane] = r < K && lane < n ? (double)gu[r * N + lane] : 0.0;
+    for (; first < last; first += step * kDmmaBlocks)
     {
-        double av[2], bv[4];
-#pragma unroll
-        for (int mi = 0; mi < 2; ++mi)
-            av[mi] = sa[(wm + mi * 8 + g) * lda + kk + qq];
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni)
-            bv[ni] = sb[(kk + qq) * kLd64 + wn + ni * 8 + g];
-#pragma unroll
-        for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-            for (int ni = 0; ni < 4; ++ni)
-                dmma_8x8x4(acc[mi][ni][0], acc[mi][ni][1], av[mi], bv[ni]);
+        const int cnt = min(kDmmaBlocks, (last - first + step - 1) / step);
+        __syncthreads(); // the places are free
+        if (tid < cnt)
+        {
+            const int i = first + tid * step;
+            const int64_t e = e0 + i + (skip >= 0 && i >= skip), ba = S.lcol_blk[e];
+            const int32_t t = S.lcol_row[e];
+            s_m[tid] = S.size[t];
+            s_a[tid] = S.blk_off[ba];
+            // row t mostly goes on as the pivot's does
+            s_c[tid] = S.blk_off[find_near(S.cols, S.row_ptr[t], S.row_ptr[t + 1], c, ba + 1 + j)] + col0;
+        }
+        __syncthreads(); // also: the strip is staged
+        // the blocks' 16-row slices go round the warps
+        int at = 0;
+        for (int b = 0; b < cnt; ++b)
+        {
+            const int M = s_m[b], ns = (M + 15) / 16;
+            const T *ga = slab + s_a[b];
+            T *gc = slab + s_c[b];
+            for (int s = (warp - at) & (kDmmaThreads / 32 - 1); s < ns; s += kDmmaThreads / 32)
+                switch (nt)
+                {
+                case 1:
+                    dmma_slice<1>(ga, gc, 16 * s, M, N, n, K, sb);
+                    break;
+                case 2:
+                    dmma_slice<2>(ga, gc, 16 * s, M, N, n, K, sb);
+                    break;
+                case 3:
+                    dmma_slice<3>(ga, gc, 16 * s, M, N, n, K, sb);
+                    break;
+                default:
+                    dmma_slice<4>(ga, gc, 16 * s, M, N, n, K, sb);
+                }
+            at += ns;
+        }
     }
-#pragma unroll
-    for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-            for (int e = 0; e < 2; ++e)
-            {
-                const int r = wm + mi * 8 + g, cc = wn + ni * 8 + 2 * qq + e;
-                if (r < mt && cc < nt)
-                    gc[(int64_t)r * N + cc] = (T)acc[mi][ni][e];
-            }
 }
 
 // Update of a level whose pivots share target rows: one CTA per listed target, its

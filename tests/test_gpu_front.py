@@ -142,3 +142,45 @@ def test_tensor_core_pivots_on_both_sides_of_the_rule(gpu, n):
     for row, ref in zip(_factors(ns, mat), first):
         for got, want in zip(row, ref):
             assert np.array_equal(got, want)
+
+
+# edges of the FP64 tensor-pipe update: slices of 16 rows, strips of 32 columns, steps of 8 and 16 of the
+# contraction (pivots of up to 128 rows), odd row lengths; rows and columns alone (lookahead) and whole levels
+@pytest.mark.parametrize("m", [1, 7, 8, 9, 16, 17, 24, 31, 33, 65, 128])
+@pytest.mark.parametrize("lookahead", [True, False])
+def test_generic_update_on_the_tensor_pipe_matches_oracle(gpu, m, lookahead):
+    mat = _dense_blocks([m, 33, 100, 1, m, 15, 64, 31], seed=200 + m)
+    osys = O.OracleSystem.from_csr(mat.sizes, mat.row_ptr, mat.cols, mat.vals)
+    osys.decompose()
+    ns = gpu.NativeSystem.from_matrix(mat)
+    ns.set_option(gpu.OPTION_UPDATE_KERNEL, 2)
+    ns.set_lookahead(lookahead)
+    ns.decompose(gpu.FP64)
+    f64 = _factors(ns, mat)
+    for i, row in enumerate(f64):
+        for c, got in enumerate(row):
+            assert rel_err(got, osys.get_block(i, c)) < 1e-12, (i, c)
+    # FP32 factors: every stored value is rounded once per pivot that updates it, seven times at most
+    ns.set_option(gpu.OPTION_BLOCK_SCALING, 0)
+    ns.decompose(gpu.MIXED)
+    for row, ref in zip(_factors(ns, mat), f64):
+        for got, want in zip(row, ref):
+            assert rel_err(got, want) < 1e-4
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+def test_tensor_pipe_update_does_not_depend_on_lookahead(gpu, prec):
+    """The update of the next pivot's row and column rounds as the rest of the update does, whether a
+    launch of its own makes it (blocks of more than 64 rows) or the pivot's kernel."""
+    for sizes in ([9, 30, 17, 64, 5, 33], [9, 30, 65, 17, 100, 5, 33]):
+        mat = _dense_blocks(sizes, seed=7)
+        got = []
+        for lookahead in (True, False):
+            ns = gpu.NativeSystem.from_matrix(mat)
+            ns.set_option(gpu.OPTION_UPDATE_KERNEL, 2)
+            ns.set_lookahead(lookahead)
+            ns.decompose(gpu.FP64 if prec == 0 else gpu.MIXED)
+            got.append(_factors(ns, mat))
+        for a, b in zip(*got):
+            for x, y in zip(a, b):
+                assert np.array_equal(x, y)
