@@ -1331,10 +1331,14 @@ int launch_flow(hyb_system *h, const T *slab, T *y, hyb::Tagged<T> *scr, int tag
     int64_t groups = (int64_t)(kFwd ? S.fwd_item_p.size() : S.bwd_item_p.size()), withhold = kFwd ? h->withhold_slot : -1;
     int mp = max_pivot(S), *status = h->d_solve_status;
     uint64_t wait_ns = h->wait_ns;
-    // CTAs for the late items (two blocks each) and for the groups (up to eight), in proportion to their
-    // blocks, but with at least an eighth of the CTAs for either kind
+    // CTAs for the late items (up to two blocks each) and for the groups (up to eight), at least an eighth
+    // for either kind. On a chain (few pivots per level) late CTAs are what shortens a hop -- they
+    // prepare the next pivots meanwhile -- and count double; with many pivots per level the groups
+    // keep the SMs busy. Solves with late:group weights 1:4, 1:2, 1:1, 2:1, 4:1: 40x40 p=8 FP64 8.4, 7.7, 7.3, 7.1,
+    // 7.7 ms, 32x32 of orders 2..10 9.7, 9.2, 8.9, 8.8, 9.2 ms; 24 mixed systems 29.3, 27.2, 30.0, 38.4, 56.5 ms.
     const int64_t ctas = (int64_t)per_sm * sm_count();
-    int64_t want = ctas * 2 * S.n / (2 * S.n + 8 * groups);
+    const bool chain = S.n < 8 * S.n_levels;
+    int64_t want = chain ? ctas * 2 * S.n / (2 * S.n + groups) : ctas * S.n / (S.n + 2 * groups);
     want = std::min(S.n, std::max(std::min(want, ctas - ctas / 8), ctas / 8));
     int late = (int)(groups == 0 ? std::min(S.n, ctas) : std::max<int64_t>(1, want));
     const unsigned grid = (unsigned)(late + std::min(groups, ctas - late));
