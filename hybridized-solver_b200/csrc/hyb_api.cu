@@ -887,7 +887,7 @@ int enqueue_generic_update(hyb_system *h, T *slab, int64_t l, cudaStream_t st, i
         int64_t cols = upper, shares = (slices + 2 * kWarps - 1) / (2 * kWarps);
         if (upper * strips * shares < hyb::kDmmaCtas * sm_count())
             shares = (slices + kWarps - 1) / kWarps;
-        shares = std::max<int64_t>(1, std::min(shares, lower));
+        shares = std::max<int64_t>(1, std::min({shares, lower, (int64_t)65535}));
         if (mode == 1)
         {
             shares = lower;
@@ -995,6 +995,11 @@ template <typename T> bool needs_tuning(const hyb_system *h)
     return false;
 }
 
+// Rounds of CTAs that a launch of k_update64_f64 keeps at least when a CTA takes two targets. Whole
+// factorizations with one and with two per CTA: 64x64 p=8 (3,969 targets per level) 440 and 421 ms, 24x24 (529)
+// 17.7 and 18.4 ms; four and eight at 64x64 438 and 489 ms, since the next pivot's CTAs wait for theirs to end.
+constexpr int kUpd64Rounds = 3;
+
 // Schur-complement updates of level l: mode 0 all of them, 1 / 2 the lookahead split.
 template <typename T> int enqueue_update(hyb_system *h, T *slab, int64_t l, cudaStream_t st, int mode,
                                          uint64_t &launches)
@@ -1028,15 +1033,20 @@ template <typename T> int enqueue_update(hyb_system *h, T *slab, int64_t l, cuda
         {
             // FP64 MMA instruction shape (HYB_OPTION_FP64_MMA_SHAPE); every shape applies the
             // same products, only the grouping of the K sums inside an instruction differs
-            if (h->fp64_shape == 2)
-                hyb::k_update64_f64<2><<<(unsigned)nu, hyb::kUpd64Threads, hyb::kUpd64Smem, st>>>(
-                    ds, slab, p0, p1, mode, sh.la_i0, sh.la_j0, h->d_status, reverse);
-            else if (h->fp64_shape == 1)
-                hyb::k_update64_f64<1><<<(unsigned)nu, hyb::kUpd64Threads, hyb::kUpd64Smem, st>>>(
-                    ds, slab, p0, p1, mode, sh.la_i0, sh.la_j0, h->d_status, reverse);
-            else
-                hyb::k_update64_f64<0><<<(unsigned)nu, hyb::kUpd64Threads, hyb::kUpd64Smem, st>>>(
-                    ds, slab, p0, p1, mode, sh.la_i0, sh.la_j0, h->d_status, reverse);
+            const int64_t upper = S.trsm_pref[p1] - S.trsm_pref[p0];
+            int64_t lower = 0; // of any pivot
+            for (int64_t p = p0; p < p1; ++p)
+                lower = std::max(lower, S.lcol_ptr[S.piv[p] + 1] - S.lcol_ptr[S.piv[p]]);
+            const int batch = (int)std::clamp<int64_t>(nu / (kUpd64Rounds * hyb::kUpd64Ctas * sm_count()), 1, hyb::kUpd64Batch);
+            const int64_t batches = (lower + batch - 1) / batch;
+            const int64_t cols = upper - (mode == 2 && sh.la_j0 >= 0);
+            const unsigned grid = (unsigned)(mode == 1 ? (sh.la_i0 >= 0 ? upper : 0) + (sh.la_j0 >= 0 ? batches : 0)
+                                                       : cols * batches);
+            auto kernel = h->fp64_shape == 2   ? hyb::k_update64_f64<2>
+                          : h->fp64_shape == 1 ? hyb::k_update64_f64<1>
+                                               : hyb::k_update64_f64<0>;
+            kernel<<<grid, hyb::kUpd64Threads, hyb::kUpd64Smem, st>>>(ds, slab, p0, p1, mode, sh.la_i0, sh.la_j0,
+                                                                      (unsigned)cols, batch, h->d_status, reverse);
             ++launches;
             HYB_LAUNCHED("k_update64_f64", l);
             return HYB_SUCCESS;

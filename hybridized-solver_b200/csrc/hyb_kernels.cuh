@@ -1321,137 +1321,196 @@ __device__ __forceinline__ void dmma_16x8x16(double &d0, double &d1, double &d2,
 
 constexpr int kLd64 = 68; // padded shared-memory row (doubles): conflict-free fragment reads
 constexpr int kUpd64Threads = 256;
+constexpr int kUpd64Ctas = 3;   // per SM
+constexpr int kUpd64Batch = 2;  // most targets of a CTA
 constexpr int kUpd64Smem = 2 * 64 * kLd64 * 8 + 16;
 
-// Uniform-64 FP64 update, the dominant work of a mesh factorization: one CTA per target
-// block, C(64x64) -= A(t,k) * U(k,c). A and U arrive by 128 bulk row copies into padded
-// shared memory while the CTA reads C into DMMA accumulator fragments; eight warps each
-// own a 16x32 eighth of C (8 m8n8k4 tiles), the K loop fully unrolled. Eight warps per CTA
+// Uniform-64 FP64 update, the dominant work of a mesh factorization: C(64x64) -= A(t,k) * U(k,c). A CTA
+// keeps U(k,c) in padded shared memory and takes `batch` rows t of the pivot's lower column in turn: A
+// arrives by 64 bulk row copies while the CTA reads C into DMMA accumulator fragments; eight warps
+// each own a 16x32 eighth of C (8 m8n8k4 tiles), the K loop fully unrolled. Eight warps per CTA
 // (24 per SM at 3 CTAs) hide the shared-memory operand latency better than four (7% less
 // FP64 factorization time at 96x96) and better than sixteen (smaller tiles, more loads
-// per DMMA). Work units as in k_update.
+// per DMMA). Alone, 3,969 targets take 93 us: 22 of the 37 TFLOP/s of the FP64 tensor pipe. The places of
+// a CTA's blocks cost five dependent loads (the target's column is guessed from the pivot's row); with divisions for
+// its indices and a search by a warp, at one target per CTA, factorizations took 20.0 ms at 24x24 p=8 (17.7 now)
+// and 439 ms at 64x64 (421 now). Two buffers of A and the next C in registers, two CTAs per SM: 18.9 and
+// 435 ms.
 // kShape: 0 m8n8k4, 1 m16n8k8, 2 m16n8k16 (FP64 MMA instruction shape; same tiling).
+// Units: per batch of the lower blocks the `cols` upper blocks of the level's pivots. Of a single pivot, in
+// mode 2 without the upper block j0 and the lower block i0, in mode 1 those alone: the blocks of row i0
+// (if any), then the batches of column j0 (if any).
 template <int kShape>
-__global__ void __launch_bounds__(kUpd64Threads)
-    k_update64_f64(DevSym S, double *__restrict__ slab, int64_t p0, int64_t p1, int mode, int i0, int j0,
-                   int *status, int reverse)
+__global__ void __launch_bounds__(kUpd64Threads, kUpd64Ctas)
+    k_update64_f64(DevSym S, double *__restrict__ slab, int64_t p0, int64_t p1, int mode, int i0, int j0, unsigned cols,
+                   int batch, int *status, int reverse)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int s_abort;
+    __shared__ int64_t s_a[kUpd64Batch], s_c[kUpd64Batch];
     double *sa = reinterpret_cast<double *>(smem_raw);
     double *sb = sa + 64 * kLd64;
     uint64_t *bar = reinterpret_cast<uint64_t *>(sb + 64 * kLd64);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
     // reverse: units in descending order, so the CTAs scheduled first at this level take the
     // targets the previous level's last CTAs wrote (still in L2)
-    const UpdUnit w = update_unit(S, p0, p1, mode, i0, j0, reverse ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
-    const int64_t li = w.li, bu = w.bu;
-    const int32_t t = S.lcol_row[li];
-    const int32_t c = S.cols[bu];
-    const int64_t tgt = warp_find_col(S.cols, S.row_ptr[t], S.row_ptr[t + 1], c);
-    const double *ga = slab + S.blk_off[S.lcol_blk[li]];
-    const double *gb = slab + S.blk_off[bu];
-    double *gc = slab + S.blk_off[tgt];
-
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    __shared__ int s_abort;
+    const unsigned unit = reverse ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
+    int64_t p = p0, j = mode == 1 ? unit : unit % cols;
+    int first = (int)(unit / cols) * batch, skip = -1;
+    if (mode == 0)
+    {
+        const int64_t u = S.trsm_pref[p0] + j;
+        p = warp_find_owner(S.trsm_pref, p0, p1, u);
+        j = u - S.trsm_pref[p];
+    }
+    const int64_t k = S.piv[p], b0 = S.diag_pos[k] + 1, e0 = S.lcol_ptr[k];
+    int last = (int)(S.lcol_ptr[k + 1] - e0);
+    if (mode == 1)
+    {
+        const int64_t n_up = i0 >= 0 ? S.row_ptr[k + 1] - b0 : 0;
+        if (j < n_up)
+        {
+            first = i0;
+            last = i0 + 1;
+        }
+        else
+        {
+            first = (int)(j - n_up) * batch;
+            skip = i0;
+            j = j0;
+        }
+    }
+    else if (mode == 2)
+    {
+        j += j0 >= 0 && j >= j0;
+        skip = i0;
+    }
+    last = min(last - (skip >= 0), first + batch);
+    const int cnt = last - first; // at most kUpd64Batch
+    if (cnt <= 0)
+        return;
+    const int64_t bu = b0 + j;
     if (tid == 0)
     {
         s_abort = schedule_aborted(status);
-        if (!s_abort)
-        {
-            mbar_init(bar, 1);
-            mbar_expect_tx(bar, 2 * 64 * 64 * 8);
-        }
+        mbar_init(bar, 1);
+    }
+    if (tid < cnt)
+    {
+        const int i = first + tid;
+        const int64_t e = e0 + i + (skip >= 0 && i >= skip), ba = S.lcol_blk[e];
+        const int32_t t = S.lcol_row[e], c = S.cols[bu];
+        s_a[tid] = S.blk_off[ba];
+        // row t mostly goes on as the pivot's does
+        s_c[tid] = S.blk_off[find_near(S.cols, S.row_ptr[t], S.row_ptr[t + 1], c, ba + 1 + j)];
     }
     __syncthreads();
     if (s_abort)
         return;
-    if (warp == 0)
-    {
-        // 64 rows of A and 64 rows of U, 512 bytes each, two per lane
+    // 64 rows of A (and, first, of U), 512 bytes each, two per lane
+    auto fetch = [&](int b) {
+        if (warp != 0)
+            return;
+        if (lane == 0)
+            mbar_expect_tx(bar, (b == 0 ? 2 : 1) * 64 * 64 * 8);
+        __syncwarp();
+        const double *ga = slab + s_a[b], *gb = slab + S.blk_off[bu];
         for (int r = lane; r < 64; r += 32)
         {
             bulk_g2s(sa + r * kLd64, ga + r * 64, 512, bar);
-            bulk_g2s(sb + r * kLd64, gb + r * 64, 512, bar);
+            if (b == 0)
+                bulk_g2s(sb + r * kLd64, gb + r * 64, 512, bar);
         }
-    }
+    };
+    fetch(0);
     const int g = lane >> 2, q = lane & 3;
     const int wm = (warp >> 1) * 16, wn = (warp & 1) * 32;
-    double acc[2][4][2];
-#pragma unroll
-    for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni)
-        {
-            const double2 v = *reinterpret_cast<const double2 *>(gc + (wm + mi * 8 + g) * 64 + wn + ni * 8 + 2 * q);
-            acc[mi][ni][0] = v.x;
-            acc[mi][ni][1] = v.y;
-        }
-    if (!mbar_wait(bar, 0))
+    for (int b = 0; b < cnt; ++b)
     {
-        if (lane == 0)
-            atomicOr(status + ST_TIMEOUT, 1);
-        // The CTA must not leave while its bulk copies can still write its shared memory:
-        // keep draining (the copies read valid global memory and complete), up to
-        // kDrainWaits further limits so the wait stays bounded.
-        for (int w = 0; w < kDrainWaits && !mbar_wait(bar, 0); ++w)
-        {
-        }
-        return;
-    }
-    if constexpr (kShape == 0)
-    {
+        double *gc = slab + s_c[b] + (wm + g) * 64 + wn + 2 * q;
+        double acc[2][4][2];
 #pragma unroll
-        for (int kk = 0; kk < 64; kk += 4)
-        {
-            double av[2], bv[4];
-#pragma unroll
-            for (int mi = 0; mi < 2; ++mi)
-                av[mi] = -sa[(wm + mi * 8 + g) * kLd64 + kk + q];
+        for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
             for (int ni = 0; ni < 4; ++ni)
-                bv[ni] = sb[(kk + q) * kLd64 + wn + ni * 8 + g];
+            {
+                const double2 v = *reinterpret_cast<const double2 *>(gc + mi * 512 + ni * 8);
+                acc[mi][ni][0] = v.x;
+                acc[mi][ni][1] = v.y;
+            }
+        if (!mbar_wait(bar, b & 1))
+        {
+            if (lane == 0)
+                atomicOr(status + ST_TIMEOUT, 1);
+            // The CTA must not leave while its bulk copies can still write its shared memory:
+            // keep draining (the copies read valid global memory and complete), up to
+            // kDrainWaits further limits so the wait stays bounded.
+            for (int w = 0; w < kDrainWaits && !mbar_wait(bar, b & 1); ++w)
+            {
+            }
+            s_abort = 1;
+        }
+        if constexpr (kShape == 0)
+        {
 #pragma unroll
-            for (int mi = 0; mi < 2; ++mi)
+            for (int kk = 0; kk < 64; kk += 4)
+            {
+                double av[2], bv[4];
+#pragma unroll
+                for (int mi = 0; mi < 2; ++mi)
+                    av[mi] = -sa[(wm + mi * 8 + g) * kLd64 + kk + q];
 #pragma unroll
                 for (int ni = 0; ni < 4; ++ni)
-                    dmma_8x8x4(acc[mi][ni][0], acc[mi][ni][1], av[mi], bv[ni]);
-        }
-    }
-    else
-    {
-        constexpr int KS = kShape == 1 ? 8 : 16; // k per instruction
+                    bv[ni] = sb[(kk + q) * kLd64 + wn + ni * 8 + g];
 #pragma unroll
-        for (int kk = 0; kk < 64; kk += KS)
-        {
-            double av[KS / 2], bv[4][KS / 4];
+                for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
-            for (int j = 0; j < KS / 4; ++j)
-            {
-                av[2 * j] = -sa[(wm + g) * kLd64 + kk + 4 * j + q];
-                av[2 * j + 1] = -sa[(wm + 8 + g) * kLd64 + kk + 4 * j + q];
+                    for (int ni = 0; ni < 4; ++ni)
+                        dmma_8x8x4(acc[mi][ni][0], acc[mi][ni][1], av[mi], bv[ni]);
             }
+        }
+        else
+        {
+            constexpr int KS = kShape == 1 ? 8 : 16; // k per instruction
 #pragma unroll
-            for (int ni = 0; ni < 4; ++ni)
+            for (int kk = 0; kk < 64; kk += KS)
+            {
+                double av[KS / 2], bv[4][KS / 4];
 #pragma unroll
                 for (int j = 0; j < KS / 4; ++j)
-                    bv[ni][j] = sb[(kk + 4 * j + q) * kLd64 + wn + ni * 8 + g];
+                {
+                    av[2 * j] = -sa[(wm + g) * kLd64 + kk + 4 * j + q];
+                    av[2 * j + 1] = -sa[(wm + 8 + g) * kLd64 + kk + 4 * j + q];
+                }
 #pragma unroll
-            for (int ni = 0; ni < 4; ++ni)
-            {
-                if constexpr (kShape == 1)
-                    dmma_16x8x8(acc[0][ni][0], acc[0][ni][1], acc[1][ni][0], acc[1][ni][1], av, bv[ni][0], bv[ni][1]);
-                else
-                    dmma_16x8x16(acc[0][ni][0], acc[0][ni][1], acc[1][ni][0], acc[1][ni][1], av, bv[ni]);
+                for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+                    for (int j = 0; j < KS / 4; ++j)
+                        bv[ni][j] = sb[(kk + 4 * j + q) * kLd64 + wn + ni * 8 + g];
+#pragma unroll
+                for (int ni = 0; ni < 4; ++ni)
+                {
+                    if constexpr (kShape == 1)
+                        dmma_16x8x8(acc[0][ni][0], acc[0][ni][1], acc[1][ni][0], acc[1][ni][1], av, bv[ni][0], bv[ni][1]);
+                    else
+                        dmma_16x8x16(acc[0][ni][0], acc[0][ni][1], acc[1][ni][0], acc[1][ni][1], av, bv[ni]);
+                }
             }
         }
+        if (b + 1 < cnt)
+        {
+            __syncthreads(); // every warp has read A
+            if (s_abort)
+                return;
+            fetch(b + 1);
+        }
+#pragma unroll
+        for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+            for (int ni = 0; ni < 4; ++ni)
+                *reinterpret_cast<double2 *>(gc + mi * 512 + ni * 8) = make_double2(acc[mi][ni][0], acc[mi][ni][1]);
     }
-#pragma unroll
-    for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni)
-            *reinterpret_cast<double2 *>(gc + (wm + mi * 8 + g) * 64 + wn + ni * 8 + 2 * q) =
-                make_double2(acc[mi][ni][0], acc[mi][ni][1]);
 }
 
 // Generic-size Schur update on the FP64 tensor pipe (DMMA m8n8k4), for blocks of any size and pivots of up

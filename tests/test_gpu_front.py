@@ -184,3 +184,30 @@ def test_tensor_pipe_update_does_not_depend_on_lookahead(gpu, prec):
         for a, b in zip(*got):
             for x, y in zip(a, b):
                 assert np.array_equal(x, y)
+
+
+# one and two targets per CTA of the 64-row FP64 update; whole levels, rows and columns alone, odd batches
+@pytest.mark.parametrize("n", [2, 3, 8, 54, 55])
+@pytest.mark.parametrize("lookahead", [True, False])
+def test_uniform_fp64_update_on_both_sides_of_the_batch_rule(gpu, n, lookahead):
+    mat = _dense_blocks([64] * n, seed=300 + n)
+    ns = gpu.NativeSystem.from_matrix(mat)
+    ns.set_lookahead(lookahead)
+    ns.decompose(gpu.FP64)
+    dense = np.vstack([np.hstack([ns.get_block(i, c, (64, 64)) for c in range(n)]) for i in range(n)])
+    # block LU with unscaled lower blocks: A = (L D^-1) D (I + U), D the pivots' own LU factors
+    a = np.zeros_like(dense)
+    off = np.concatenate([[0], np.cumsum(mat.sizes)])
+    full = O.OracleSystem.from_csr(mat.sizes, mat.row_ptr, mat.cols, mat.vals)
+    for i in range(n):
+        for c in range(n):
+            a[off[i] : off[i + 1], off[c] : off[c + 1]] = full.get_block(i, c)
+    low, up = np.zeros_like(dense), np.eye(64 * n)
+    for i in range(n):
+        r = slice(64 * i, 64 * i + 64)
+        low[r, : 64 * i] = dense[r, : 64 * i]
+        d = dense[r, r]
+        low[r, r] = (np.tril(d, -1) + np.eye(64)) @ np.triu(d)
+        up[r, 64 * i + 64 :] = dense[r, 64 * i + 64 :]
+    # 64 n products of a row and a column, each rounded to 2^-53
+    assert rel_err(low @ up, a) < 64 * n * 2.0**-53
