@@ -174,7 +174,7 @@ struct hyb_system
     bool block_scaling = true;            // HYB_OPTION_BLOCK_SCALING (mixed form)
     bool alternate_walk = true;           // HYB_OPTION_ALTERNATE_WALK
     int pair_passes = 1;                  // HYB_OPTION_PAIR_PASSES (mixed form; 2: inner update launched apart)
-    int row_pivots = -1;                  // HYB_OPTION_ROW_PIVOTS: -1 per precision (mixed 2, FP64 0)
+    int row_pivots = -1;                  // HYB_OPTION_ROW_PIVOTS: -1 k_front, or 2 (kFrontTcMax)
     int update_sm_reserve = 4;            // HYB_OPTION_UPDATE_SM_RESERVE
     // generic-size Schur updates: HYB_OPTION_UPDATE_KERNEL (-1: tuned per size bucket), and
     // the tuned choice per precision and bucket (-1: not tuned yet)
@@ -198,7 +198,7 @@ struct hyb_system
     // level-parity halves of fused_half slots of 64 x 64 doubles
     double *d_piv64f = nullptr;
     int64_t fused_half = 0;
-    int lu_once = -1; // HYB_OPTION_PIVOT_LU_ONCE: -1 per precision (FP64 once, mixed fused)
+    int lu_once = -1; // HYB_OPTION_PIVOT_LU_ONCE: -1 k_front
     int fp64_shape = 1; // HYB_OPTION_FP64_MMA_SHAPE (m16n8k8: 0.6% faster than m8n8k4 at 128x128 p=8)
     // independent systems stacked in one handle (hyb_system_set_segments): unknown offsets,
     // their device copy, norms per segment and column, and the last solve's results

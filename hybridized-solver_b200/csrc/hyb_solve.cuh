@@ -17,8 +17,8 @@
 //  - the other ("early") blocks go in groups of up to eight to a CTA each, which adds their products in
 //    registers as the sources arrive; the group nearest the pivot collects the others' sums.
 // Measured on a B200, both directions, one right-hand side, before (flags, D_k substituted on the chain) and
-// after: 40x40 p=8 FP64 21.9 to 8.5 ms, 64x64 56 to 23.5 ms, 16x16 p=4 2.3 to 1.1 ms; two FP32
-// solves of a mixed step at 31x31 16.2 to 8.3 ms, at 96x96 169 to 105 ms. Of a hop's 1.8 us about
+// after: 40x40 p=8 FP64 21.9 to 7.1 ms, 64x64 56 to 19.9 ms, 16x16 p=4 2.3 to 1.0 ms; two FP32
+// solves of a mixed step at 31x31 16.2 to 6.9 ms, at 96x96 169 to 91.7 ms. Of a hop's 1.8 us about
 // 0.4 us is the trip through L2, 0.95 us the additions, their reduction and the stores.
 //
 // Two forms with the same arithmetic (bit-identical results): k_flow, one cooperative launch per

@@ -217,10 +217,10 @@ typedef enum
     HYB_OPTION_UPDATE_KERNEL = 11,
     /* Pivots of 33-64 rows: 1 factors each diagonal block once and then solves its row's
      * upper blocks from the stored factors (two launches); 0: one fused launch in which every
-     * CTA of a pivot factors the block itself before its strip; -1 (default): 1 for the FP64
-     * form (its LU is costly and the redundant copies slow the concurrent update), 0 for the
-     * mixed form (its FP32 LU is cheap and the extra launch lengthens the pivot chain). All
-     * give the same factors. */
+     * CTA of a pivot factors the block itself before its strip; -1 (default): the kernel that
+     * takes pivots of all sizes up to 128 rows (FP64 inside, with the update by the pivot
+     * before it where it can; mixed levels with many upper blocks take HYB_OPTION_ROW_PIVOTS
+     * 2 instead). 0 and 1 give the same factors; -1 differs from them by rounding. */
     HYB_OPTION_PIVOT_LU_ONCE = 12,
     /* FP64 MMA instruction shape of the FP64 form's 64-block Schur update: 0 m8n8k4,
      * 1 (default) m16n8k8, 2 m16n8k16. The same products, summed in different groups inside
@@ -246,7 +246,8 @@ typedef enum
      * each pivot is factored once and inverted (blocked triangular inverses), and its
      * upper blocks are taken as products with the inverse, so the pivot's critical path
      * holds no substitution (FP32 factors that differ from 0 and 1 by rounding); -1
-     * (default): 2 for the mixed form, 0 for the FP64 form. */
+     * (default): 2 on the mixed form's tensor-core levels with more than 44 upper blocks per
+     * pivot, else the kernel of HYB_OPTION_PIVOT_LU_ONCE -1. */
     HYB_OPTION_ROW_PIVOTS = 15,
     /* Mixed form, two-pivot passes: SMs the main update launch leaves free for the next
      * unit's pivot work, which runs beside it (default 4, at most 64). The pivot chain is
